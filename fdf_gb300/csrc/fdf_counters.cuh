@@ -12,7 +12,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 
 // Per-thread counts stay far below 2^32 within one launch; the block sums are 64-bit.
 struct LocCounts {
-  unsigned int lost = 0, oob = 0, evals = 0, done = 0, lost_total = 0, fb = 0;
+  unsigned int lost = 0, oob = 0, evals = 0, done = 0, lost_total = 0;
   unsigned int err = 0;
 };
 
@@ -39,26 +39,29 @@ __device__ __forceinline__ unsigned int warp_histogram_rank(unsigned int hkey, u
 // Adds the block's counters to cnt.  Every thread of the block calls it (blockDim.x a
 // multiple of 32, at most 1024).
 __device__ __forceinline__ void block_flush_counts(const LocCounts &m, DevCounters *cnt) {
-  __shared__ unsigned long long red[32][6];
+  __shared__ unsigned int red[32][5];
   __shared__ unsigned int rerr[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();   // a previous call's readers are done with the shared words
-  unsigned long long v[6] = {m.lost, m.oob, m.evals, m.done, m.lost_total, m.fb};   // widened before the sums
+  // one REDUX per counter: a warp's sums stay below 2^32 (at most MAX_TRAVERSAL evaluations per
+  // particle, and no thread walks more than a few thousand particles in one launch)
+  unsigned int v[5] = {m.lost, m.oob, m.evals, m.done, m.lost_total};
 #pragma unroll
-  for (int q = 0; q < 6; ++q) v[q] = warp_sum_u64(v[q]);
+  for (int q = 0; q < 5; ++q) v[q] = __reduce_add_sync(0xffffffffu, v[q]);
   const unsigned int e = __reduce_or_sync(0xffffffffu, m.err);
   if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < 6; ++q) red[w][q] = v[q];
+    for (int q = 0; q < 5; ++q) red[w][q] = v[q];
     rerr[w] = e;
   }
   __syncthreads();
-  if (threadIdx.x < 7) {
+  if (threadIdx.x < 6) {
     const int q = threadIdx.x;
-    if (q < 6) {
+    if (q < 5) {
       unsigned long long t = 0;
       for (int k = 0; k < nw; ++k) t += red[k][q];
-      // slot q of this block's flush row (CNT_LOST .. CNT_FB are 0 .. 5, the order of v[])
+      // slot q of this block's flush row (CNT_LOST .. CNT_LOST_TOTAL are 0 .. 4, the order of v[]; the
+      // walk adds its rare fallbacks to CNT_FB itself)
       if (t) atomicAdd(&cnt->stripes[blockIdx.x & (FDF_CNT_STRIPES - 1)][q], t);
     } else {
       unsigned int t = 0;

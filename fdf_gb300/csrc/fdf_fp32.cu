@@ -23,8 +23,8 @@ using fdfx::mul;
 using fdfx::sub;
 
 // One 128-B FP32 row per cell (the layout and the error bound are in fdf_walk.cuh): the first
-// vertex c0 as a float pair, thr32, the absolute slack for the FP64 arithmetic of the table, then
-// per face n32 = fl32(n) and e32 = fl32(n . (fc - c0)).
+// vertex c0 as a float pair, the two margins, then per face n32 = fl32(n) and
+// e32 = fl32(n . (fc - c0)).
 __global__ void k_build_table32(const double *__restrict__ planes, const double *__restrict__ coor, GridDims g,
                                 float *__restrict__ table) {
   const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -34,35 +34,43 @@ __global__ void k_build_table32(const double *__restrict__ planes, const double 
   const double *v0 = coor + 3 * (((long long)k * (g.JM + 1) + j) * (long long)(g.IM + 1) + i);
   const double *row = planes + c * FDF_ROW;
   float *t = table + c * FDF_ROW32;
-  double c0[3];
+  const unsigned int sw = row32_swizzle((unsigned int)c);
+  float *h0 = t + 4 * sw, *h1 = t + 4 * (1u ^ sw);
+  double c0[3], size = 0.0;
   for (int q = 0; q < 3; ++q) {
     const float h = __double2float_rn(v0[q]);
     const float l = __double2float_rn(sub(v0[q], (double)h));
-    t[q] = h;
-    t[4 + q] = l;
+    h0[q] = h;
+    h1[q] = l;
     c0[q] = add((double)h, (double)l);   // exact: the pair's value
+    size = add(size, fabs((double)h));
   }
-  const double thr = row[36];
-  // rounded up with a little headroom: thr32 * (1 - 2^-24)^2 >= thr, which the error bound uses;
-  // a degenerate cell carries the sign bit
-  float thr32 = __double2float_ru(mul(thr, 1.0 + 0x1p-22));
-  if (fdfx::ubits(row[37]) != 0ULL) thr32 = -fabsf(thr32) - 1.0f;
-  t[3] = thr32;
   double sigma = 0.0;   // max over faces of sum_i |fc_i - c0_i| |n_i|
+  bool wide = false;    // a value the FP32 bound does not cover: every face goes to FP64
   for (int f = 0; f < 6; ++f) {
     const double *p = row + 6 * f;
     const double dx = sub(p[0], c0[0]), dy = sub(p[1], c0[1]), dz = sub(p[2], c0[2]);
     const double e = add(add(mul(dx, p[3]), mul(dy, p[4])), mul(dz, p[5]));
     const double sg = add(add(mul(fabs(dx), fabs(p[3])), mul(fabs(dy), fabs(p[4]))), mul(fabs(dz), fabs(p[5])));
     sigma = sg > sigma ? sg : sigma;
-    float *o = t + 8 + 4 * f;
+    wide = wide || !(fabs(e) <= 0x1p100) || !(sg <= 0x1p100);
+    float *o = t + 4 * ((2u + f) ^ sw);
     o[0] = __double2float_rn(p[3]);
     o[1] = __double2float_rn(p[4]);
     o[2] = __double2float_rn(p[5]);
     o[3] = __double2float_rn(e);
   }
+  // The faces' own margin: thr rounded up with a little headroom (thr32 (1 - 2^-24)^2 >= thr), and
   // the FP64 roundings of e and of the reference's own distance, 32 eps sigma (rounded up)
-  t[7] = __double2float_ru(mul(sigma, 0x1p-48));
+  h1[3] = fabsf(__fadd_rn(__double2float_ru(mul(row[36], 1.0 + 0x1p-22)), __double2float_ru(mul(sigma, 0x1p-48))));
+  // The cell's: the same with headroom for its own roundings, and the row's part of 40 u sum_i ex_i
+  const double slack = add(mul(sigma, 0x1p-48), mul(size, 40.0 * 0x1p-48));
+  const float base = __double2float_ru(mul(add(row[36], slack), 1.0 + 0x1p-19));
+  if (fdfx::ubits(row[37]) != 0ULL) {   // a degenerate cell
+    h1[3] = -1.0f;
+    wide = true;
+  }
+  h0[3] = wide ? __int_as_float(0x7f800000) : base;
 }
 
 // (hi, lo) float pair held in a double slot of the swarm arrays
@@ -84,8 +92,7 @@ __device__ __forceinline__ float2 pair_add(float2 p, float v) {
 
 // Writes the located (or LOST) particle: weights (UpdateParticleWeights in FP32: clamp
 // d <= 1e-14, then the three ratios), cell and status.
-__device__ __forceinline__ void store_located32(const SwarmBuf &b, int s, const GridDims &g, bool lost, int i, int j,
-                                                int k, float (&dv)[6]) {
+__device__ __forceinline__ void store_located32(const SwarmBuf &b, int s, int cell, bool lost, float (&dv)[6]) {
   if (lost) {
     b.cell[s] = -1;
     b.status[s] = ST_LOST;
@@ -97,7 +104,7 @@ __device__ __forceinline__ void store_located32(const SwarmBuf &b, int s, const 
   b.a1f[s] = __fdiv_rn(dv[F_LEFT], __fadd_rn(dv[F_LEFT], dv[F_RIGHT]));
   b.a2f[s] = __fdiv_rn(dv[F_BOTTOM], __fadd_rn(dv[F_BOTTOM], dv[F_TOP]));
   b.a3f[s] = __fdiv_rn(dv[F_BACK], __fadd_rn(dv[F_FRONT], dv[F_BACK]));
-  b.cell[s] = (int)(((long long)k * g.JM + j) * g.IM + i);
+  b.cell[s] = cell;
   b.status[s] = ST_ACTIVE_AND_LOCATED;
 }
 
@@ -130,23 +137,8 @@ __device__ __forceinline__ unsigned int settle_key32(bool lost, int cell, float2
   return key;
 }
 
-// How far past the previous cell a particle is, in cells, from the first evaluation's
-// distances: for each index direction with a negative face, -d_neg / (d_lower + d_upper)
-// (the two planes' distances add up to the cell's width there).  Only steers which exact path
-// the learned form takes, so it may be approximate; a degenerate width gives +inf.
-__device__ __forceinline__ float beyond_cells(const float (&dv)[6]) {
-  float far = 0.f;
-  const int lo[3] = {F_LEFT, F_BOTTOM, F_BACK}, hi[3] = {F_RIGHT, F_TOP, F_FRONT};
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const float dl = dv[lo[a]], dh = dv[hi[a]], width = dl + dh;
-    const float neg = dl < 0.f ? -dl : (dh < 0.f ? -dh : 0.f);
-    if (neg > 0.f) far = fmaxf(far, width > 0.f ? __fdividef(neg, width) : INFINITY);
-  }
-  return far;
-}
-
 // Advect + locate, one thread per particle.
+//   FAR: the walks may start far from the particles (walk_ref32).
 //   FIRST == false: the reference walk from the previous cell (or cell (0,0,0)).
 //   FIRST == true:  the reference's first evaluation, in the previous cell; a particle that it
 //                   does not conclude and that lies at least far_cells past that cell is
@@ -155,7 +147,7 @@ __device__ __forceinline__ float beyond_cells(const float (&dv)[6]) {
 //                   walk's second cell, and finished by k_locate32_path (its key and
 //                   histogram entry are written there); a nearer one continues the reference
 //                   walk here.
-template <bool FIRST>
+template <bool FIRST, bool FAR>
 __global__ void __launch_bounds__(FDF_LOC_THREADS, FDF_LOC_MIN_BLOCKS) k_locate32(SwarmBuf b, GridDims g, const float *__restrict__ table,
                                                   const double *__restrict__ planes, float dt32, int advect,
                                                   int reset_first, const double *__restrict__ bbox,
@@ -184,34 +176,21 @@ __global__ void __launch_bounds__(FDF_LOC_THREADS, FDF_LOC_MIN_BLOCKS) k_locate3
     bool lost = false;
     if (st != ST_ACTIVE_AND_LOCATED) {
       Walk32 w;
-      w.i = 0; w.j = 0; w.k = 0; w.err = 0u;
+      w.i = 0; w.j = 0; w.k = 0;
       if (cell >= 0 && (long long)cell < g.Nc) cell_ijk(g, (unsigned int)cell, w.i, w.j, w.k);
-      walk_ref32(table, planes, g, px, py, pz, FIRST ? 1 : FDF_MAX_TRAVERSAL, w, m.fb);
-      m.err |= w.err;
-      m.done += (unsigned int)w.evaluated;
-      // learned form: the walk's next cell (w.i, w.j, k) is where the reference continues;
-      // outside the grid it ends there as LOST, as the reference's next loop test does
-      const bool next_inside = w.i >= 0 && w.i < g.IM && w.j >= 0 && w.j < g.JM && w.k >= 0 && w.k < g.KM;
-      if (FIRST && !w.concluded && !w.lost && next_inside && !(far_cells <= beyond_cells(w.e.dv))) {
-        // close to the previous cell: the reference walk continues here from its second cell
-        Walk32 w2;
-        w2.i = w.i; w2.j = w.j; w2.k = w.k; w2.err = 0u;
-        walk_ref32(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL - 1, w2, m.fb);
-        m.err |= w2.err;
-        m.done += (unsigned int)w2.evaluated;
-        m.evals += (unsigned int)(w.evaluated + w2.evaluated);
-        lost = w2.lost || !w2.concluded;
-        store_located32(b, s, g, lost, w2.i, w2.j, w2.k, w2.e.dv);
-        cell = lost ? -1 : (int)(((long long)w2.k * g.JM + w2.j) * g.IM + w2.i);
-      } else if (FIRST && !w.concluded && !w.lost && next_inside) {
-        wait = true;
-        m.evals += (unsigned int)w.evaluated;
-        b.cell[s] = (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
+      walk_ref32<false, false, FIRST, FAR>(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL, w, cnt, 0.0, 0.0, 0.0, nullptr,
+                                      far_cells);
+      if (w.degenerate) m.err |= ERRBIT_DEGENERATE;
+      m.done += w.evaluated();
+      m.evals += FIRST ? w.evaluated() : (unsigned int)(w.cycle ? FDF_MAX_TRAVERSAL : w.steps);
+      wait = FIRST && w.wait;
+      const int at = (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
+      if (wait) {
+        b.cell[s] = at;   // P1, where the walk continues
       } else {
-        m.evals += FIRST ? (unsigned int)w.evaluated : (unsigned int)(w.cycle ? FDF_MAX_TRAVERSAL : w.steps);
         lost = w.lost || !w.concluded;
-        store_located32(b, s, g, lost, w.i, w.j, w.k, w.e.dv);
-        cell = lost ? -1 : (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
+        store_located32(b, s, at, lost, w.dv);
+        cell = lost ? -1 : at;
       }
     } else {
       lost = (cell < 0);
@@ -274,38 +253,37 @@ __global__ void __launch_bounds__(FDF_GUESS_THREADS, FDF_GUESS_MIN_BLOCKS) k_loc
                                                         unsigned int *__restrict__ count, unsigned int sentinel,
                                                         const unsigned int *__restrict__ pending,
                                                         const int *__restrict__ guess, int lookahead) {
-  const long long npend = (long long)cnt->pending;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
+  const unsigned int npend = (unsigned int)cnt->pending;   // at most FDF_MAX_PARTICLES = 2^29
+  const unsigned int stride = gridDim.x * blockDim.x;
+  const unsigned int lane = threadIdx.x & 31;
   unsigned int pev = 0, hits = 0;
   LocCounts m;
-  for (long long base = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); base < npend; base += stride) {
-    const long long t = base + lane;
+  for (unsigned int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < npend; base += stride) {
+    const unsigned int t = base + lane;
     unsigned int hkey = 0xffffffffu;
     int s = 0;
     if (t < npend) {
       s = (int)pending[t];
       const float2 px = ld_pair(b.x, s), py = ld_pair(b.y, s), pz = ld_pair(b.z, s);
       Walk32 w;
-      w.err = 0u;
       cell_ijk(g, (unsigned int)b.cell[s], w.i, w.j, w.k);
       int gi, gj, gk;
       cell_ijk(g, (unsigned int)guess[t], gi, gj, gk);
       // P1 and the guess lie in the grid, so does every cell of the path between them
       for (int q = 1; q <= lookahead; ++q) {
         const int ci = path_index(w.i, gi, q), cj = path_index(w.j, gj, q), ck = path_index(w.k, gk, q);
-        prefetch_row_l1(table + (((long long)ck * g.JM + cj) * g.IM + ci) * FDF_ROW32);
+        prefetch_row_l1(table + (size_t)(((unsigned int)ck * g.JM + cj) * g.IM + ci) * FDF_ROW32);
         if (ci == gi && cj == gj && ck == gk) break;   // the predicted path has reached the guess
       }
-      walk_ref32<false, true>(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL - 1, w, m.fb, 0.0, 0.0, 0.0, gi, gj,
-                              gk, &hits);
-      m.err |= w.err;
-      m.done += (unsigned int)w.evaluated;
-      m.evals += (unsigned int)w.evaluated;
-      pev += (unsigned int)w.evaluated;
+      Path32 path{w.i, w.j, w.k, gi, gj, gk, 0u};
+      walk_ref32<false, true>(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL - 1, w, cnt, 0.0, 0.0, 0.0, &path);
+      hits += path.hits;
+      if (w.degenerate) m.err |= ERRBIT_DEGENERATE;
+      pev += w.evaluated();
       const bool lost = w.lost || !w.concluded;
-      store_located32(b, s, g, lost, w.i, w.j, w.k, w.e.dv);
-      const int cell = lost ? -1 : (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
+      const int at = (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
+      store_located32(b, s, at, lost, w.dv);
+      const int cell = lost ? -1 : at;
       const unsigned int key =
           settle_key32(lost, cell, px, py, pz, drop_removed, bbox, fbox, sentinel, m.lost, m.oob, m.lost_total);
       keys[s] = key;
@@ -315,6 +293,7 @@ __global__ void __launch_bounds__(FDF_GUESS_THREADS, FDF_GUESS_MIN_BLOCKS) k_loc
     const unsigned int r = warp_histogram_rank(hkey, count);
     if (hkey != 0xffffffffu) rank[s] = r;
   }
+  m.done = m.evals = pev;
   block_flush_counts(m, cnt);
   block_add_u64(hits, &cnt->guess_taken_total);
   block_add_u64(pev, &cnt->guess_evals_total);
@@ -756,14 +735,15 @@ void launch_locate32(const SwarmBuf &b, int n_cap, GridDims g, const float *tabl
                      unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
                      unsigned int *pending, float far_cells, cudaStream_t s) {
   constexpr int th = FDF_LOC_THREADS;
-  if (pending)
-    k_locate32<true><<<blocks_for(n_cap, th), th, 0, s>>>(b, g, table, planes, (float)dt, advect, drop_removed, bbox,
-                                                          fbox, drop_removed, cnt, keys, rank, count, sentinel,
-                                                          pending, n_cap, far_cells);
-  else
-    k_locate32<false><<<blocks_for(n_cap, th), th, 0, s>>>(b, g, table, planes, (float)dt, advect, drop_removed,
-                                                           bbox, fbox, drop_removed, cnt, keys, rank, count, sentinel,
-                                                           nullptr, n_cap, 0.f);
+  auto go = [&](auto kernel, unsigned int *pend, float far) {
+    kernel<<<blocks_for(n_cap, th), th, 0, s>>>(b, g, table, planes, (float)dt, advect, drop_removed, bbox, fbox,
+                                                drop_removed, cnt, keys, rank, count, sentinel, pend, n_cap, far);
+  };
+  // without the advection the particles come from anywhere (the initial setup's corner start)
+  if (pending && advect) go(k_locate32<true, false>, pending, far_cells);
+  else if (pending) go(k_locate32<true, true>, pending, far_cells);
+  else if (advect) go(k_locate32<false, false>, nullptr, 0.f);
+  else go(k_locate32<false, true>, nullptr, 0.f);
 }
 
 void launch_compact_pending(const unsigned int *scan, int n_cap, unsigned int *list, DevCounters *cnt,

@@ -106,6 +106,9 @@ struct GridDims {
   FastDiv fIM, fJM, fMX, fMY;   // by IM, JM (cells) and IM+1, JM+1 (nodes)
 };
 
+// The 16-byte chunk q of cell c's FP32 plane-table row is stored at position q ^ row32_swizzle(c).
+__host__ __device__ __forceinline__ unsigned int row32_swizzle(unsigned int c) { return (c * 0x9E3779B1u) >> 29; }
+
 // cell id -> (i, j, k)
 __device__ __forceinline__ void cell_ijk(const GridDims &g, unsigned int c, int &i, int &j, int &k) {
   unsigned int t = g.fIM.div(c);
@@ -125,18 +128,17 @@ __device__ __forceinline__ void node_ijk(const GridDims &g, unsigned int q, int 
 
 // Threads per block of the advect + locate kernels.  A block keeps its SM slot until its
 // slowest walk ends, so smaller blocks waste fewer warp slots on the walk-length tail (FP32 walk
-// per 64M-particle step at 1152 resident threads: 3.15 ms in 64-thread blocks, 3.17 in 128, 3.18
-// in 96, 3.42 in 256).
+// per 64M-particle step at 1024 resident threads: 2.32 ms in 64-thread blocks, 2.34 in 128, 2.30 in
+// 32; the learned first pass 2.37, 2.39, 2.37).
 #ifndef FDF_LOC_THREADS
 #define FDF_LOC_THREADS 64
 #endif
-// Resident blocks per SM the FP32 locate kernels are compiled for.  The walk is bound by load
-// latency, so resident threads beat spills up to a point: with 176-B plane-table rows 1024
-// threads (64 registers) beat 768 (80): 3.9 against 4.8 ms per 64M-particle step, and 1280 (48
-// registers) spilled too much; with the 128-B rows 1152 threads (56 registers, a few more spills)
-// take 3.17 against 3.22 ms for the FP32 walk.
+// Resident blocks per SM the FP32 locate kernels are compiled for: 1024 threads leave 64 registers,
+// the most threads without a spill in the walk's loop (per 64M-particle step 2.30 ms; 2.45 at 1152
+// threads and 2.68 at 1280, whose spills go through the L1 data pipe that the row loads need; 2.66 at
+// 896, 2.90 at 768).
 #ifndef FDF_LOC_MIN_BLOCKS
-#define FDF_LOC_MIN_BLOCKS (1152 / FDF_LOC_THREADS)
+#define FDF_LOC_MIN_BLOCKS (1024 / FDF_LOC_THREADS)
 #endif
 // Resident blocks per SM of the plain walk (its steps decided from the FP32 table; per
 // 64M-particle step 1024 resident threads take 7.6 ms against 8.6 ms at 768 and 8.4 ms at 1280
@@ -153,7 +155,7 @@ __device__ __forceinline__ void node_ijk(const GridDims &g, unsigned int q, int 
 #define FDF_ORDER_MIN_BLOCKS 8
 #endif
 // Resident 256-thread blocks per SM the learned form's walk from P1 is compiled for (4: 64
-// registers, 0.701 ms per 64M-particle step against 0.712 ms at 3 with 80 registers).
+// registers, 0.52 ms per 64M-particle step against 0.55 ms at 3 with 80 registers).
 #ifndef FDF_GUESS_MIN_BLOCKS
 #define FDF_GUESS_MIN_BLOCKS 4
 #endif

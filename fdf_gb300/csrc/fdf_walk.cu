@@ -73,12 +73,12 @@ __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
         return fdfx::split_rn(v);
       };
       Walk32 w;
-      w.i = 0; w.j = 0; w.k = 0; w.err = 0u;   // InitializeTraversalParameters: previous cell, else (0,0,0)
+      w.i = 0; w.j = 0; w.k = 0;   // InitializeTraversalParameters: previous cell, else (0,0,0)
       if (cell >= 0 && (long long)cell < g.Nc) cell_ijk(g, (unsigned int)cell, w.i, w.j, w.k);
-      walk_ref32<true>(table, planes, g, split(x), split(y), split(z), FDF_MAX_TRAVERSAL, w, m.fb, x, y, z);
-      m.err |= w.err;
+      walk_ref32<true, false, false, true>(table, planes, g, split(x), split(y), split(z), FDF_MAX_TRAVERSAL, w, cnt, x, y, z);
+      if (w.degenerate) m.err |= ERRBIT_DEGENERATE;
       m.evals += (unsigned int)(w.cycle ? FDF_MAX_TRAVERSAL : w.steps);
-      m.done += (unsigned int)w.evaluated;
+      m.done += w.evaluated();
       if (w.lost || !w.concluded) {
         lost = true;
         cell = -1;

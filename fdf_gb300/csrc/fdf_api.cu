@@ -710,7 +710,8 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
                        ctx->perm, s);
   // the plain form orders each cell by PID (the oracle's summation order); the precision forms
   // keep each cell's particles in their previous order (no gather of the PIDs)
-  launch_order_segments(ctx->cell_start, (int)(g.Nc + 1), f32 ? nullptr : src.pid, ctx->perm, s);
+  ctx->launches += launch_order_segments(ctx->cell_start, (int)g.Nc, f32 ? nullptr : src.pid, ctx->perm,
+                                         drop ? nullptr : ctx->rank, ctx->cap, s) - 1;
   size_t e2 = prof ? record_event(ctx, s) : 0;
   if (!locate_only) CU(cudaStreamWaitEvent(s, ctx->ev_corner, 0));
   size_t e3 = prof ? record_event(ctx, s) : 0;
@@ -791,7 +792,8 @@ int resort(FdfContext *ctx, int remove_lost, int remove_oob, int64_t *removed_lo
                      ctx->keys, ctx->rank, ctx->cell_start, ctx->sentinel, s);
   exclusive_scan_u32(ctx->cell_start, g.Nc + 2, ctx->scan_sums, s);
   launch_scatter_slots(ctx->keys, ctx->rank, ctx->cap, ctx->cnt, ctx->sentinel, 1, ctx->cell_start, ctx->perm, s);
-  launch_order_segments(ctx->cell_start, (int)(g.Nc + 1), f32 ? nullptr : src.pid, ctx->perm, s);
+  ctx->launches += launch_order_segments(ctx->cell_start, (int)g.Nc, f32 ? nullptr : src.pid, ctx->perm, ctx->rank,
+                                         ctx->cap, s) - 1;
   if (f32)
     launch_gather_interp32(src, dst, ctx->cap, g, ctx->corner32, ctx->perm, ctx->cell_start, ctx->cnt, s, GATHER_COPY);
   else

@@ -207,8 +207,10 @@ void exclusive_scan_u32(unsigned int *data, long long count, unsigned int *sums,
 void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, int n_cap, const DevCounters *cnt,
                           unsigned int sentinel, int keep_lost, const unsigned int *cell_start, unsigned int *perm,
                           cudaStream_t s);
-void launch_order_segments(const unsigned int *cell_start, int nseg, const long long *pid, unsigned int *perm,
-                           cudaStream_t s);
+// Orders every cell's slots by (PID, previous slot), or by previous slot when pid is null; with
+// lost_scratch [n_cap], also the LOST particles' bucket ncells.  Returns the kernels launched.
+int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
+                           unsigned int *lost_scratch, int n_cap, cudaStream_t s);
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
                           unsigned int *cell_start, unsigned int *cursor, unsigned int *sums, cudaStream_t s);
 

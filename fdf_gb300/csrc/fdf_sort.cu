@@ -16,6 +16,8 @@
 //      input, and no gather of the PIDs), as does the standalone sort.
 #include "fdf_internal.cuh"
 
+#include <algorithm>
+
 namespace {
 
 // ---- exclusive scan of a u32 array (reduce -> scan of block sums -> scan with offsets) ----
@@ -147,113 +149,303 @@ __global__ void __launch_bounds__(256) k_scatter_slots(const unsigned int *__res
     if (keep[q]) perm[start[q] + rk[q]] = (unsigned int)(base + (long long)q * blockDim.x);
 }
 
-// Orders every cell's slots by (PID, previous slot) -- or by previous slot alone when
-// pid is null.  Segments are short (a few particles per cell on average): up to 8 entries
-// are checked and, when out of order, sorted in registers by a 19-comparator sorting
-// network; longer ones are insertion-sorted in place in global memory.
-constexpr int SEG_NET = 8;
+// Orders every cell's slots by (PID, previous slot), or by previous slot alone: the keys are then
+// the slots themselves, one 32-bit word per entry and no gather.  One thread per cell; a cell's
+// entries decide who works on it:
+//   up to 8    its thread: a 19-comparator sorting network in registers (two or four cells per
+//              thread, their loads issued first, measured no faster);
+//   9 to 32    its warp, one lane per entry (two cells at a time up to 16): a bitonic network of
+//              shuffles, the next cells' entries already loading;
+//   33 to 128  its warp, in shared memory;
+//   above      its block, together: in shared memory (up to SEG_SHARED entries) or in place in
+//              global memory.
+// (A thread's own insertion sort in global memory, which the cells above 8 took before, is a chain of
+// dependent loads.  Sort stage per step, before -> now: 64M particles, 4.5 per cell, by slot
+// 0.51 -> 0.45 ms, by PID 1.28 -> 1.17 ms; 32M particles, 27 per cell, 0.49 -> 0.34 and
+// 1.60 -> 0.65 ms.)
+constexpr int SEG_NET = 8, SEG_WARP = 128, SEG_SHARED = 1024;
 
-__device__ __forceinline__ bool key_gt(long long ka, unsigned int va, long long kb, unsigned int vb) {
-  return ka > kb || (ka == kb && va > vb);
+// The key of slot v: its PID and then the slot, or the slot alone.
+template <bool PID>
+struct SlotKey {
+  long long pid;
+  unsigned int slot;
+  __device__ __forceinline__ bool after(const SlotKey &o) const { return pid > o.pid || (pid == o.pid && slot > o.slot); }
+};
+template <>
+struct SlotKey<false> {
+  unsigned int slot;
+  __device__ __forceinline__ bool after(const SlotKey &o) const { return slot > o.slot; }
+};
+template <bool PID>
+__device__ __forceinline__ SlotKey<PID> slot_key(unsigned int v, const long long *__restrict__ pid) {
+  SlotKey<PID> k;
+  if constexpr (PID) k.pid = __ldg(pid + v);
+  k.slot = v;
+  return k;
 }
 
-// One cell's slots [s0, s0 + L) ordered by (key, previous slot), key = PID or, with pid null,
-// the previous slot itself.
-__device__ __forceinline__ void order_cell(unsigned int s0, unsigned int L, const long long *__restrict__ pid,
-                                           unsigned int *__restrict__ perm) {
-  if (L < 2) return;
-  if (L <= SEG_NET) {
-    long long kp[SEG_NET];
-    unsigned int ix[SEG_NET];
+template <bool PID>
+__device__ __forceinline__ SlotKey<PID> last_key() {   // sorts after every slot's (slots are below 2^31)
+  SlotKey<PID> k;
+  if constexpr (PID) k.pid = 0x7fffffffffffffffLL;
+  k.slot = 0xffffffffu;
+  return k;
+}
+
+// Ascending bitonic sort of the n items that get(i) reads and set(i, item) writes, by `many` threads
+// of which this is number `me`: the form whose comparators all point the same way, so that the
+// items past n of the next power of two need not exist.
+template <typename Get, typename Set, typename Sync>
+__device__ __forceinline__ void bitonic(unsigned int n, unsigned int me, unsigned int many, Get get, Set set,
+                                        Sync sync) {
+  unsigned int P = 1;
+  while (P < n) P <<= 1;
+  auto exchange = [&](unsigned int i, unsigned int j) {
+    if (j >= n) return;
+    const auto x = get(i), y = get(j);
+    if (x.after(y)) {
+      set(i, y);
+      set(j, x);
+    }
+  };
+  for (unsigned int h = 2; h <= P; h <<= 1) {
+    for (unsigned int t = me; t < P / 2; t += many) {   // mirrored halves of each h items
+      const unsigned int o = t & (h / 2 - 1), q = 2 * (t - o);
+      exchange(q + o, q + h - 1 - o);
+    }
+    sync();
+    for (unsigned int d = h / 4; d >= 1; d >>= 1) {
+      for (unsigned int t = me; t < P / 2; t += many) {
+        const unsigned int o = t & (d - 1), q = 2 * (t - o);
+        exchange(q + o, q + o + d);
+      }
+      sync();
+    }
+  }
+}
+template <typename Get, typename Set>
+__device__ __forceinline__ void block_bitonic(unsigned int n, Get get, Set set) {
+  bitonic(n, threadIdx.x, blockDim.x, get, set, [] { __syncthreads(); });
+}
+
+// One key per lane, ascending within each group of W lanes.
+template <int W, bool PID>
+__device__ __forceinline__ void lane_bitonic(SlotKey<PID> &k, int lane) {
+#pragma unroll
+  for (int h = 2; h <= W; h <<= 1)
+#pragma unroll
+    for (int d = h >> 1; d > 0; d >>= 1) {
+      SlotKey<PID> o;
+      o.slot = __shfl_xor_sync(0xffffffffu, k.slot, d);
+      if constexpr (PID) o.pid = __shfl_xor_sync(0xffffffffu, k.pid, d);
+      const bool up = h == W || (lane & h) == 0, low = (lane & d) == 0;
+      if constexpr (PID) {
+        if (k.after(o) == (up == low)) k = o;   // equal keys only among the padding
+      } else {
+        k.slot = up == low ? min(k.slot, o.slot) : max(k.slot, o.slot);
+      }
+    }
+}
+
+// The cells of `todo` (a lane mask; each lane holds its own cell's start s0 and length L <= W),
+// 32 / W at a time.
+template <int W, bool PID>
+__device__ __forceinline__ void order_lanes(unsigned int todo, unsigned int s0, unsigned int L, int lane,
+                                            const long long *__restrict__ pid, unsigned int *__restrict__ perm) {
+  const int group = lane / W, at = lane % W;
+  unsigned int q0 = 0u, n = 0u, v = 0u;
+  // takes this group's next cell out of `todo` and starts loading its entries
+  auto take = [&](unsigned int &q, unsigned int &m, unsigned int &e) {
+    unsigned int mine = 0u;
+#pragma unroll
+    for (int g = 0; g < 32 / W; ++g) {
+      if (g == group) mine = todo;
+      todo &= todo - 1u;   // 0 stays 0
+    }
+    const int who = mine ? __ffs((int)mine) - 1 : 0;
+    q = __shfl_sync(0xffffffffu, s0, who);
+    m = __shfl_sync(0xffffffffu, L, who);
+    if (!mine) m = 0u;
+    e = at < (int)m ? perm[q + at] : 0u;
+  };
+  take(q0, n, v);
+  while (__any_sync(0xffffffffu, n != 0u)) {
+    SlotKey<PID> k = at < (int)n ? slot_key<PID>(v, pid) : last_key<PID>();
+    const unsigned int w0 = q0, wn = n, was = v;
+    take(q0, n, v);
+    lane_bitonic<W, PID>(k, lane);
+    if (at < (int)wn && k.slot != was) perm[w0 + at] = k.slot;
+  }
+}
+
+template <bool PID>
+__global__ void __launch_bounds__(256, FDF_ORDER_MIN_BLOCKS) k_order_segments(const unsigned int *__restrict__ cell_start,
+                                                                             int nseg,
+                                                                             const long long *__restrict__ pid,
+                                                                             unsigned int *__restrict__ perm) {
+  using Key = SlotKey<PID>;
+  __shared__ unsigned int big[256][2], nbig;
+  __shared__ Key item[SEG_SHARED];
+  static_assert(SEG_SHARED == 8 * SEG_WARP, "one warp's part each, or the block's");
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  unsigned int s0 = 0u, L = 0u;
+  if (c < nseg) {
+    s0 = cell_start[c];
+    L = cell_start[c + 1] - s0;
+  }
+  if (L >= 2u && L <= (unsigned int)SEG_NET) {
+    Key k[SEG_NET];
     bool sorted = true;
 #pragma unroll
-    for (int q = 0; q < SEG_NET; ++q) {
-      // padding (max, max) sorts after every real entry (slots are below 2^31)
-      kp[q] = 0x7fffffffffffffffLL;
-      ix[q] = 0xffffffffu;
-      if (q < (int)L) {
-        ix[q] = perm[s0 + q];
-        kp[q] = pid ? pid[ix[q]] : (long long)ix[q];
-        if (q > 0 && key_gt(kp[q - 1], ix[q - 1], kp[q], ix[q])) sorted = false;
+    for (int e = 0; e < SEG_NET; ++e) {
+      k[e] = last_key<PID>();
+      if (e < (int)L) {
+        k[e] = slot_key<PID>(perm[s0 + e], pid);
+        if (e > 0 && k[e - 1].after(k[e])) sorted = false;
       }
     }
-    if (sorted) return;
-    auto cx = [&](int a, int b) {
-      const bool sw = key_gt(kp[a], ix[a], kp[b], ix[b]);
-      const long long ka = sw ? kp[b] : kp[a], kb = sw ? kp[a] : kp[b];
-      const unsigned int va = sw ? ix[b] : ix[a], vb = sw ? ix[a] : ix[b];
-      kp[a] = ka; kp[b] = kb; ix[a] = va; ix[b] = vb;
-    };
-    cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
-    cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
-    cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
-    cx(2, 4); cx(3, 5);
-    cx(1, 4); cx(3, 6);
-    cx(1, 2); cx(3, 4); cx(5, 6);
+    if (!sorted) {
+      auto cx = [&](int a, int b) {
+        const Key x = k[a], y = k[b];
+        if constexpr (PID) {
+          const bool sw = x.after(y);
+          k[a] = sw ? y : x;
+          k[b] = sw ? x : y;
+        } else {
+          k[a].slot = min(x.slot, y.slot);
+          k[b].slot = max(x.slot, y.slot);
+        }
+      };
+      cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
+      cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
+      cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
+      cx(2, 4); cx(3, 5);
+      cx(1, 4); cx(3, 6);
+      cx(1, 2); cx(3, 4); cx(5, 6);
 #pragma unroll
-    for (int q = 0; q < SEG_NET; ++q)
-      if (q < (int)L) perm[s0 + q] = ix[q];
-  } else {
-    for (unsigned int q = 1; q < L; ++q) {
-      unsigned int v = perm[s0 + q];
-      long long kv = pid ? pid[v] : (long long)v;
-      unsigned int r = q;
-      while (r > 0) {
-        unsigned int u = perm[s0 + r - 1];
-        long long ku = pid ? pid[u] : (long long)u;
-        if (ku < kv || (ku == kv && u < v)) break;
-        perm[s0 + r] = u;
-        --r;
-      }
-      perm[s0 + r] = v;
+      for (int e = 0; e < SEG_NET; ++e)
+        if (e < (int)L) perm[s0 + e] = k[e].slot;
+    }
+  }
+  const unsigned int w16 = __ballot_sync(0xffffffffu, L > (unsigned int)SEG_NET && L <= 16u);
+  const unsigned int w32 = __ballot_sync(0xffffffffu, L > 16u && L <= 32u);
+  if (w16) order_lanes<16, PID>(w16, s0, L, lane, pid, perm);
+  if (w32) order_lanes<32, PID>(w32, s0, L, lane, pid, perm);
+  for (unsigned int todo = __ballot_sync(0xffffffffu, L > 32u && L <= (unsigned int)SEG_WARP); todo; todo &= todo - 1u) {
+    const int who = __ffs((int)todo) - 1;
+    const unsigned int q0 = __shfl_sync(0xffffffffu, s0, who), n = __shfl_sync(0xffffffffu, L, who);
+    Key *mine = item + (threadIdx.x >> 5) * SEG_WARP;
+    for (unsigned int e = lane; e < n; e += 32) mine[e] = slot_key<PID>(perm[q0 + e], pid);
+    __syncwarp();
+    bitonic(n, (unsigned int)lane, 32u, [&](unsigned int i) { return mine[i]; },
+            [&](unsigned int i, const Key &x) { mine[i] = x; }, [] { __syncwarp(); });
+    for (unsigned int e = lane; e < n; e += 32) perm[q0 + e] = mine[e].slot;
+    __syncwarp();
+  }
+  if (threadIdx.x == 0) nbig = 0u;
+  if (!__syncthreads_or(L > (unsigned int)SEG_WARP)) return;
+  if (L > (unsigned int)SEG_WARP) {
+    const unsigned int at = atomicAdd(&nbig, 1u);   // any order: each cell is sorted by itself
+    big[at][0] = s0;
+    big[at][1] = L;
+  }
+  __syncthreads();
+  const unsigned int many = nbig;
+  for (unsigned int q = 0; q < many; ++q) {
+    const unsigned int q0 = big[q][0], n = big[q][1];
+    if (n <= (unsigned int)SEG_SHARED) {
+      for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) item[e] = slot_key<PID>(perm[q0 + e], pid);
+      __syncthreads();
+      block_bitonic(n, [&](unsigned int i) { return item[i]; }, [&](unsigned int i, const Key &v) { item[i] = v; });
+      for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) perm[q0 + e] = item[e].slot;
+      __syncthreads();
+    } else {
+      block_bitonic(n, [&](unsigned int i) { return slot_key<PID>(perm[q0 + i], pid); },
+                    [&](unsigned int i, const Key &v) { perm[q0 + i] = v.slot; });
     }
   }
 }
 
-__global__ void __launch_bounds__(256, FDF_ORDER_MIN_BLOCKS) k_order_segments(const unsigned int *__restrict__ cell_start, int nseg,
-                                                       const long long *__restrict__ pid,
-                                                       unsigned int *__restrict__ perm) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nseg) return;
-  const unsigned int s0 = cell_start[c];
-  order_cell(s0, cell_start[c + 1] - s0, pid, perm);
+// The LOST particles that the initial setup and the staged calls keep: one bucket, which may hold a
+// few percent of the swarm, ordered like the cells' slots but by the whole GPU.  Chunks of
+// LOST_CHUNK entries are sorted in shared memory, then neighbouring runs are merged, twice as long
+// each time, between perm and `other`: every entry finds its rank in the partner run by binary
+// search.  The host knows only the swarm's capacity, so the merges it cannot rule out are launched
+// and return at once (1.5 us each).  (A single thread's insertion sort took 0.40 s for the 20,000
+// LOST of 1M particles on the sinusoidal 64x64x1024 grid, 0.94 s for the 78,000 of 6M on 96x96x1536.)
+constexpr int LOST_CHUNK = 2048, LOST_THREADS = 1024;
+
+template <bool PID>
+__global__ void __launch_bounds__(LOST_THREADS) k_lost_chunks(const unsigned int *__restrict__ bucket,
+                                                             const long long *__restrict__ pid,
+                                                             unsigned int *__restrict__ perm) {
+  using Key = SlotKey<PID>;
+  __shared__ Key item[LOST_CHUNK];
+  const unsigned int s0 = bucket[0], L = bucket[1] - s0;
+  for (unsigned int c0 = blockIdx.x * LOST_CHUNK; c0 < L; c0 += gridDim.x * LOST_CHUNK) {
+    const unsigned int n = min(L - c0, (unsigned int)LOST_CHUNK);
+    unsigned int *run = perm + s0 + c0;
+    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) item[e] = slot_key<PID>(run[e], pid);
+    __syncthreads();
+    block_bitonic(n, [&](unsigned int i) { return item[i]; }, [&](unsigned int i, const Key &v) { item[i] = v; });
+    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) run[e] = item[e].slot;
+    __syncthreads();
+  }
 }
 
-// The order by previous slot (the precision forms and the standalone sort): the keys are the
-// slots themselves, so the sorting network compares one 32-bit word per entry (sort stage per
-// 64M-particle step 0.61 -> 0.47 ms against the general kernel with a null PID array; two or four
-// cells per thread, their loads issued first, measured no faster).
-__global__ void __launch_bounds__(256, FDF_ORDER_MIN_BLOCKS) k_order_segments_slot(
-    const unsigned int *__restrict__ cell_start, int nseg, unsigned int *__restrict__ perm) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nseg) return;
-  const unsigned int s0 = cell_start[c], L = cell_start[c + 1] - s0;
-  if (L < 2) return;
-  if (L > (unsigned int)SEG_NET) {
-    order_cell(s0, L, nullptr, perm);
+// Merges runs of `run` entries pairwise from `from` to `to` (both indexed like perm) while the
+// bucket holds more than one; last: copies the result back to `to` = perm when the merges made (one
+// per doubling of LOST_CHUNK below the bucket's length) left it in the other array.
+template <bool PID>
+__global__ void __launch_bounds__(256) k_lost_merge(const unsigned int *__restrict__ bucket,
+                                                   const long long *__restrict__ pid, unsigned int run,
+                                                   const unsigned int *__restrict__ from,
+                                                   unsigned int *__restrict__ to, int last) {
+  const unsigned int s0 = bucket[0], L = bucket[1] - s0;
+  const unsigned int stride = gridDim.x * blockDim.x;
+  if (last) {
+    int merges = 0;
+    for (unsigned long long r = LOST_CHUNK; r < L; r <<= 1) ++merges;
+    if (merges & 1)
+      for (unsigned int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += stride) to[s0 + p] = from[s0 + p];
     return;
   }
-  unsigned int ix[SEG_NET];
-  bool sorted = true;
-#pragma unroll
-  for (int e = 0; e < SEG_NET; ++e) {   // padding (max) sorts after every slot (slots are below 2^31)
-    ix[e] = e < (int)L ? perm[s0 + e] : 0xffffffffu;
-    if (e > 0 && e < (int)L && ix[e - 1] > ix[e]) sorted = false;
+  if (run >= L) return;
+  for (unsigned int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += stride) {
+    const unsigned int v = from[s0 + p];
+    const SlotKey<PID> k = slot_key<PID>(v, pid);
+    const unsigned int own = p / run * run, pair = own / (2 * run) * (2 * run);
+    unsigned int lo = own == pair ? min(own + run, L) : pair, base = lo;
+    unsigned int hi = own == pair ? min(lo + run, L) : own;
+    while (lo < hi) {   // the partner's entries before k: keys are distinct (slots differ)
+      const unsigned int mid = lo + (hi - lo) / 2;
+      if (k.after(slot_key<PID>(from[s0 + mid], pid))) lo = mid + 1;
+      else hi = mid;
+    }
+    to[s0 + pair + (p - own) + (lo - base)] = v;
   }
-  if (sorted) return;
-  auto cx = [&](int a, int b) {
-    const unsigned int va = min(ix[a], ix[b]), vb = max(ix[a], ix[b]);
-    ix[a] = va; ix[b] = vb;
-  };
-  cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
-  cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
-  cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
-  cx(2, 4); cx(3, 5);
-  cx(1, 4); cx(3, 6);
-  cx(1, 2); cx(3, 4); cx(5, 6);
-#pragma unroll
-  for (int e = 0; e < SEG_NET; ++e)
-    if (e < (int)L) perm[s0 + e] = ix[e];
+}
+
+// Returns the number of kernels launched.
+template <bool PID>
+int order_lost(const unsigned int *bucket, const long long *pid, unsigned int *perm, unsigned int *other, int n_cap,
+                cudaStream_t s) {
+  const long long chunks = ((long long)n_cap + LOST_CHUNK - 1) / LOST_CHUNK;
+  const unsigned int blocks = (unsigned int)std::min<long long>(std::max<long long>(chunks, 1), 304);
+  k_lost_chunks<PID><<<blocks, LOST_THREADS, 0, s>>>(bucket, pid, perm);
+  if (n_cap <= LOST_CHUNK) return 1;
+  int launched = 2;
+  const unsigned int *from = perm;
+  unsigned int *to = other;
+  for (long long run = LOST_CHUNK; run < n_cap; run *= 2) {
+    k_lost_merge<PID><<<4 * blocks, 256, 0, s>>>(bucket, pid, (unsigned int)run, from, to, 0);
+    from = to;
+    to = from == perm ? other : perm;
+    ++launched;
+  }
+  k_lost_merge<PID><<<4 * blocks, 256, 0, s>>>(bucket, pid, 0u, other, perm, 1);
+  return launched;
 }
 
 // count[cell[s]] += 1 for 0 <= cell[s] < ncells (warp-aggregated integer atomics)
@@ -314,16 +506,14 @@ void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, in
   k_scatter_slots<<<blocks, th, 0, s>>>(keys, rank, cnt, sentinel, keep_lost, cell_start, perm);
 }
 
-void launch_order_segments(const unsigned int *cell_start, int nseg, const long long *pid, unsigned int *perm,
-                           cudaStream_t s) {
-  const int th = 256;
-  if (pid) {
-    const int blocks = (nseg + th - 1) / th;
-    k_order_segments<<<blocks, th, 0, s>>>(cell_start, nseg, pid, perm);
-  } else {
-    const int blocks = (nseg + th - 1) / th;
-    k_order_segments_slot<<<blocks, th, 0, s>>>(cell_start, nseg, perm);
-  }
+int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
+                           unsigned int *lost_scratch, int n_cap, cudaStream_t s) {
+  const int th = 256, blocks = (ncells + th - 1) / th;
+  if (pid) k_order_segments<true><<<blocks, th, 0, s>>>(cell_start, ncells, pid, perm);
+  else k_order_segments<false><<<blocks, th, 0, s>>>(cell_start, ncells, nullptr, perm);
+  if (!lost_scratch) return 1;
+  return 1 + (pid ? order_lost<true>(cell_start + ncells, pid, perm, lost_scratch, n_cap, s)
+                  : order_lost<false>(cell_start + ncells, nullptr, perm, lost_scratch, n_cap, s));
 }
 
 // Stable counting sort of particle slots by cell id, on caller-provided scratch:
@@ -338,5 +528,5 @@ void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsign
   k_cell_histogram<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start);
   exclusive_scan_u32(cell_start, ncells + 1, sums, s);
   k_cell_slots<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start, cursor, perm);
-  launch_order_segments(cell_start, (int)ncells, nullptr, perm, s);
+  launch_order_segments(cell_start, (int)ncells, nullptr, perm, nullptr, 0, s);
 }

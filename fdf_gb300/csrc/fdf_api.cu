@@ -198,19 +198,11 @@ int fdf_SetUcat(FdfContext *ctx, const double *ucat, int node_sized) {
   if (!ctx || !ucat) return fail(ctx, FDF_ERR_ARG_NULL, "fdf_SetUcat: null argument");
   if (!ctx->has_grid) return fail(ctx, FDF_ERR_ARG_WRONGSTATE, "fdf_SetUcat: call fdf_SetGrid first");
   const GridDims &g = ctx->g;
-  // Host-side transpose to the device SoA layout [3][Nc].
-  std::vector<double> soa(3 * (size_t)g.Nc);
-  const long long mx = node_sized ? g.IM + 1 : g.IM, my = node_sized ? g.JM + 1 : g.JM;
-  for (long long k = 0; k < g.KM; ++k)
-    for (long long j = 0; j < g.JM; ++j)
-      for (long long i = 0; i < g.IM; ++i) {
-        long long c = (k * g.JM + j) * g.IM + i;
-        const double *v = ucat + 3 * ((k * my + j) * mx + i);
-        soa[c] = v[0]; soa[g.Nc + c] = v[1]; soa[2 * g.Nc + c] = v[2];
-      }
+  // to the device as it is, into the corner field's buffer (made anew from ucat whenever it is
+  // read), and there to one array per component
   CU(cudaSetDevice(ctx->device));
-  CU(cudaMemcpyAsync(ctx->ucat, soa.data(), 24ull * g.Nc, cudaMemcpyHostToDevice, ctx->stream));
-  launch_f64_to_f32(ctx->ucat, ctx->ucat32, 3 * g.Nc, ctx->stream);
+  CU(cudaMemcpyAsync(ctx->corner, ucat, 24ull * (node_sized ? g.Nn : g.Nc), cudaMemcpyHostToDevice, ctx->stream));
+  launch_ucat_in(ctx->corner, g, node_sized ? 1 : 0, ctx->ucat, ctx->ucat32, ctx->stream);
   CHECK_LAUNCH();
   ctx->launches += 1;
   CU(cudaStreamSynchronize(ctx->stream));
@@ -597,16 +589,11 @@ int fdf_GetCornerField(FdfContext *ctx, double *corner) {
   if (!ctx->has_ucat) return fail(ctx, FDF_ERR_ARG_WRONGSTATE, "fdf_GetCornerField: no ucat");
   CU(cudaSetDevice(ctx->device));
   // the step computes only the nodes next to occupied cells; the full field is made here
-  launch_center_to_corner(ctx->ucat, ctx->g, ctx->corner, nullptr, nullptr, ctx->stream);
+  launch_center_to_corner_aos(ctx->ucat, ctx->g, ctx->corner, ctx->stream);
   CHECK_LAUNCH();
   ctx->launches += 1;
-  std::vector<double> soa(3 * (size_t)ctx->g.Nn);
-  CU(cudaMemcpyAsync(soa.data(), ctx->corner, 24ull * ctx->g.Nn, cudaMemcpyDeviceToHost, ctx->stream));
+  CU(cudaMemcpyAsync(corner, ctx->corner, 24ull * ctx->g.Nn, cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  const long long Nn = ctx->g.Nn;
-  for (long long q = 0; q < Nn; ++q) {
-    corner[3 * q] = soa[q]; corner[3 * q + 1] = soa[Nn + q]; corner[3 * q + 2] = soa[2 * Nn + q];
-  }
   return FDF_SUCCESS;
 }
 
@@ -679,7 +666,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
     exclusive_scan_u32(L.pflag + nw, nw + 1, L.scan_sums, s);
     launch_compact_pending(L.pflag, ctx->cap, L.pending, ctx->cnt, s);
     eg0 = prof ? record_event(ctx, s) : 0;
-    mlp_guess_tc(L.tc_img, L.infer_bf16, L.bias, L.norm, src.x, src.y, src.z, 1, L.pending, &ctx->cnt->pending, 0,
+    mlp_guess_tc(L.tc_img, L.infer_bf16, L.bias, L.norm, src.x, src.y, src.z, 1, 1, L.pending, &ctx->cnt->pending, 0,
                  ctx->cap, g, L.guess, ctx->num_sms, &ctx->cnt->err, s);
     eg1 = prof ? record_event(ctx, s) : 0;
     launch_locate32_path(src, ctx->cap, g, ctx->table32, ctx->planes, ctx->bbox, ctx->fbox, drop, ctx->cnt,
@@ -1299,24 +1286,20 @@ int fdf_GetFaceMomentum(FdfContext *ctx, double *mi, double *mj, double *mk) {
     return fail(ctx, FDF_ERR_ARG_WRONGSTATE, "fdf_GetFaceMomentum: no momentum deposit (fdf_SetMomentumDeposit)");
   const GridDims &g = ctx->g;
   const long long nfs[3] = {(g.IM + 1LL) * g.JM * g.KM, g.IM * (g.JM + 1LL) * g.KM, (long long)g.IM * g.JM * (g.KM + 1LL)};
-  const long long nf = nfs[0] + nfs[1] + nfs[2];
   CU(cudaSetDevice(ctx->device));
-  if (form_is32(ctx->out_form)) {
-    launch_f32_to_f64(ctx->mom32, ctx->mom, 3 * nf, ctx->stream);
+  // one family at a time through the corner field's buffer (made anew whenever it is read), which
+  // holds 24 bytes for every node, and so for every face of a family
+  double *out[3] = {mi, mj, mk};
+  long long off = 0;
+  for (int fam = 0; fam < 3; ++fam) {
+    if (form_is32(ctx->out_form)) launch_vec3_out(ctx->mom32 + off, nfs[fam], ctx->corner, ctx->stream);
+    else launch_vec3_out(ctx->mom + off, nfs[fam], ctx->corner, ctx->stream);
     CHECK_LAUNCH();
     ctx->launches += 1;
+    CU(cudaMemcpyAsync(out[fam], ctx->corner, 24ull * nfs[fam], cudaMemcpyDeviceToHost, ctx->stream));
+    off += 3 * nfs[fam];
   }
-  std::vector<double> soa(3 * (size_t)nf);
-  CU(cudaMemcpyAsync(soa.data(), ctx->mom, 24ull * nf, cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  double *out[3] = {mi, mj, mk};
-  size_t off = 0;
-  for (int fam = 0; fam < 3; ++fam) {
-    const long long n = nfs[fam];
-    for (long long q = 0; q < n; ++q)
-      for (int c = 0; c < 3; ++c) out[fam][3 * q + c] = soa[off + (size_t)c * n + q];
-    off += 3 * (size_t)n;
-  }
   return FDF_SUCCESS;
 }
 

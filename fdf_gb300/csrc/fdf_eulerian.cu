@@ -469,18 +469,11 @@ int fdf_GetUcat(FdfContext *ctx, double *ucat, int node_sized) {
   if (!ctx->has_grid) return fail(ctx, FDF_ERR_ARG_WRONGSTATE, "fdf_GetUcat: call fdf_SetGrid first");
   const GridDims &g = ctx->g;
   CU(cudaSetDevice(ctx->device));
-  std::vector<double> soa(3 * (size_t)g.Nc);
-  CU(cudaMemcpyAsync(soa.data(), ctx->ucat, 24ull * g.Nc, cudaMemcpyDeviceToHost, ctx->stream));
+  launch_ucat_out(ctx->ucat, g, node_sized ? 1 : 0, ctx->corner, ctx->stream);   // (made anew whenever it is read)
+  CHECK_LAUNCH();
+  ctx->launches += 1;
+  CU(cudaMemcpyAsync(ucat, ctx->corner, 24ull * (node_sized ? g.Nn : g.Nc), cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  const long long mx = node_sized ? g.IM + 1 : g.IM, my = node_sized ? g.JM + 1 : g.JM;
-  if (node_sized) memset(ucat, 0, 24ull * g.Nn);
-  for (long long k = 0; k < g.KM; ++k)
-    for (long long j = 0; j < g.JM; ++j)
-      for (long long i = 0; i < g.IM; ++i) {
-        const long long c = (k * g.JM + j) * g.IM + i;
-        double *v = ucat + 3 * ((k * my + j) * mx + i);
-        v[0] = soa[c]; v[1] = soa[g.Nc + c]; v[2] = soa[2 * g.Nc + c];
-      }
   return FDF_SUCCESS;
 }
 

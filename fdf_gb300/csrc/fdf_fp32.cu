@@ -712,11 +712,6 @@ __global__ void __launch_bounds__(XF_TILE) k_to_host(SwarmBuf b, int n, GridDims
     tile_out(const_cast<double *>(h.f[f]) + (long long)xf_bs(f) * p0, sm + xf_off(f), xf_bs(f) * m);
 }
 
-__global__ void k_f64_to_f32(const double *__restrict__ in, float *__restrict__ out, long long n) {
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q < n) out[q] = (float)in[q];
-}
-
 __global__ void k_f32_to_f64(const float *__restrict__ in, double *__restrict__ out, long long n) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (q < n) out[q] = (double)in[q];
@@ -836,10 +831,6 @@ void launch_swarm_to_host(const SwarmBuf &b, int n, GridDims g, void *const f[7]
   const unsigned blocks = (unsigned)((n + XF_TILE - 1) / XF_TILE);
   if (f32) k_to_host<true><<<blocks, XF_TILE, 0, s>>>(b, n, g, h);
   else k_to_host<false><<<blocks, XF_TILE, 0, s>>>(b, n, g, h);
-}
-
-void launch_f64_to_f32(const double *in, float *out, long long n, cudaStream_t s) {
-  k_f64_to_f32<<<blocks_for(n, 256), 256, 0, s>>>(in, out, n);
 }
 
 void launch_f32_to_f64(const float *in, double *out, long long n, cudaStream_t s) {

@@ -176,6 +176,13 @@ void launch_build_planes(const double *coor_aos, GridDims g, double *planes, uns
 // cell_start == nullptr: every node; else only nodes adjacent to an occupied cell.
 void launch_center_to_corner(const double *ucat, GridDims g, double *corner, const unsigned int *cell_start,
                              unsigned long long *nodes_done, cudaStream_t s);
+void launch_center_to_corner_aos(const double *ucat, GridDims g, double *corner, cudaStream_t s);
+// Vector fields between the callers' [..][3] layout and the device's [3][..]: ucat in (with its FP32
+// copy) and out, cell- or node-sized; any [3][n] array out.
+void launch_ucat_in(const double *aos, GridDims g, int node_sized, double *ucat, float *ucat32, cudaStream_t s);
+void launch_ucat_out(const double *ucat, GridDims g, int node_sized, double *aos, cudaStream_t s);
+void launch_vec3_out(const double *soa, long long n, double *aos, cudaStream_t s);
+void launch_vec3_out(const float *soa, long long n, double *aos, cudaStream_t s);
 // Advect + walk.  Writes the new cell (or -1) and status in place, keys[s] = cell
 // or sentinel (LOST / removed), and histograms the kept keys into count[] (bucket
 // Nc = LOST particles, counted only when keep_lost), with rank[s] = the particle's rank
@@ -267,7 +274,6 @@ void launch_swarm_to_aos32(const SwarmBuf &b, int n, GridDims g, double *pos, do
 // 16-byte aligned; f = position, velocity, weight, P, cell, pid, status), either form.
 void launch_swarm_from_host(const void *const f[7], int n, GridDims g, const SwarmBuf &b, bool f32, cudaStream_t s);
 void launch_swarm_to_host(const SwarmBuf &b, int n, GridDims g, void *const f[7], bool f32, cudaStream_t s);
-void launch_f64_to_f32(const double *in, float *out, long long n, cudaStream_t s);
 void launch_f32_to_f64(const float *in, double *out, long long n, cudaStream_t s);
 
 // On-device volumetric seeding (fdf_seed.cu), bit-identical to the host generator.

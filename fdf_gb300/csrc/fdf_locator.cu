@@ -362,43 +362,34 @@ static int locator_predict(FdfContext *ctx, const double *position, int64_t n, i
   if (n == 0) return FDF_SUCCESS;
   CU(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  std::vector<double> soa(3 * (size_t)n);
-  for (int64_t p = 0; p < n; ++p)
-    for (int d = 0; d < 3; ++d) soa[d * (size_t)n + p] = position[3 * p + d];
-  // one buffer: positions [3][n] f64, outputs [n][3] f32, guesses [n] i32, the error word
-  const size_t off_out = 24ull * n, off_guess = off_out + (12ull * n + 255) / 256 * 256,
-               off_err = off_guess + (4ull * n + 255) / 256 * 256;
+  // one buffer: positions [n][3] f64, cells [n][3] i64, outputs [n][3] f32, the error word
+  const size_t off_cell = 24ull * n, off_out = off_cell + 24ull * n, off_err = off_out + (12ull * n + 255) / 256 * 256;
   char *mem = nullptr;
   CU(cudaMalloc((void **)&mem, off_err + 256));
   double *d_pos = (double *)mem;
+  long long *d_cell = (long long *)(mem + off_cell);
   float *d_out = (float *)(mem + off_out);
-  int *d_guess = (int *)(mem + off_guess);
   unsigned int *d_err = (unsigned int *)(mem + off_err);
-  cudaError_t e = cudaMemcpyAsync(d_pos, soa.data(), 24ull * n, cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaMemcpyAsync(d_pos, position, 24ull * n, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_err, 0, sizeof(unsigned int), s);
   if (e == cudaSuccess) {
-    mlp_guess_tc(ctx->loc.tc_img, ctx->loc.infer_bf16, ctx->loc.bias, ctx->loc.norm, d_pos, d_pos + n,
-                 d_pos + 2 * n, 0, nullptr, nullptr, (int)n, (int)n, ctx->g, d_guess, ctx->num_sms, d_err, s, d_out,
-                 stall_test);
+    mlp_guess_tc(ctx->loc.tc_img, ctx->loc.infer_bf16, ctx->loc.bias, ctx->loc.norm, d_pos, d_pos + 1, d_pos + 2, 0,
+                 3, nullptr, nullptr, (int)n, (int)n, ctx->g, nullptr, ctx->num_sms, d_err, s, d_cell,
+                 outputs ? d_out : nullptr, stall_test);
     ctx->launches += 1;
     e = cudaGetLastError();
   }
-  std::vector<int> gh((size_t)n);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(gh.data(), d_guess, 4ull * n, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess && outputs) e = cudaMemcpyAsync(outputs, d_out, 12ull * n, cudaMemcpyDeviceToHost, s);
   unsigned int errw = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&errw, d_err, 4, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && !(errw & ERRBIT_TC_TIMEOUT)) {
+    e = cudaMemcpyAsync(cell_id, d_cell, 24ull * n, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && outputs) e = cudaMemcpyAsync(outputs, d_out, 12ull * n, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
   cudaFree(mem);
   if (e != cudaSuccess) return fail(ctx, FDF_ERR_GPU, std::string("fdf_LocatorPredict: ") + cudaGetErrorString(e));
   if (errw & ERRBIT_TC_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "fdf_LocatorPredict: tensor-core wait timed out");
-  const long long IM = ctx->g.IM, JM = ctx->g.JM;
-  for (int64_t p = 0; p < n; ++p) {
-    const long long c = gh[p];
-    cell_id[3 * p] = c % IM;
-    cell_id[3 * p + 1] = (c / IM) % JM;
-    cell_id[3 * p + 2] = c / (IM * JM);
-  }
   return FDF_SUCCESS;
 }
 

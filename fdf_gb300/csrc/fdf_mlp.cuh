@@ -83,6 +83,7 @@ void mlp_init_params_host(unsigned long long seed, float *params);
 size_t mlp_tc_image_bytes();
 void mlp_pack_tc(const float *params, unsigned char *img, int bf16, cudaStream_t s);
 void mlp_guess_tc(const unsigned char *img, int bf16, const float *bias, const MlpNorm &norm, const double *x,
-                  const double *y, const double *z, int pairs, const unsigned int *list,
+                  const double *y, const double *z, int pairs, int stride, const unsigned int *list,
                   const unsigned long long *list_count, int n_host, int n_cap, GridDims g, int *guess, int num_sms,
-                  unsigned int *err, cudaStream_t s, float *yout = nullptr, int stall_test = 0);
+                  unsigned int *err, cudaStream_t s, long long *cell3 = nullptr, float *yout = nullptr,
+                  int stall_test = 0);

@@ -120,8 +120,9 @@ template <bool BF16>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_mlp_guess_tc(const unsigned char *__restrict__ wimg, const float *__restrict__ bias_g, MlpNorm norm,
                    const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ pz,
-                   int pairs, const unsigned int *__restrict__ list, const unsigned long long *__restrict__ list_count,
-                   int n_host, GridDims g, int *__restrict__ guess, float *__restrict__ yout,
+                   int pairs, int stride, const unsigned int *__restrict__ list, const unsigned long long *__restrict__ list_count,
+                   int n_host, GridDims g, int *__restrict__ guess, long long *__restrict__ cell3,
+                   float *__restrict__ yout,
                    unsigned int *__restrict__ err, unsigned long long wait_limit, int stall_test) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -226,9 +227,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   auto fetch_raw = [&](unsigned p, unsigned long long (&raw)[3]) {
     raw[0] = raw[1] = raw[2] = 0ull;
     if (p != NO_ROW) {
-      raw[0] = reinterpret_cast<const unsigned long long *>(px)[p];
-      raw[1] = reinterpret_cast<const unsigned long long *>(py)[p];
-      raw[2] = reinterpret_cast<const unsigned long long *>(pz)[p];
+      const size_t at = (size_t)p * stride;
+      raw[0] = reinterpret_cast<const unsigned long long *>(px)[at];
+      raw[1] = reinterpret_cast<const unsigned long long *>(py)[at];
+      raw[2] = reinterpret_cast<const unsigned long long *>(pz)[at];
     }
   };
   auto to_inputs = [&](unsigned p, const unsigned long long (&raw)[3], float &x, float &y, float &z) {
@@ -314,7 +316,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           const float t = (ys[d] + 1.0f) * 0.5f * (float)N[d];
           idx[d] = (t == t) ? (int)fminf(fmaxf(floorf(t), 0.f), (float)(N[d] - 1)) : 0;
         }
-        guess[r] = (idx[2] * g.JM + idx[1]) * g.IM + idx[0];
+        if (cell3) { cell3[3 * r] = idx[0]; cell3[3 * r + 1] = idx[1]; cell3[3 * r + 2] = idx[2]; }
+        else guess[r] = (idx[2] * g.JM + idx[1]) * g.IM + idx[0];
       }
     }
     to_inputs(np, nraw, cx, cy, cz);
@@ -339,9 +342,9 @@ void mlp_pack_tc(const float *params, unsigned char *img, int bf16, cudaStream_t
 }
 
 void mlp_guess_tc(const unsigned char *img, int bf16, const float *bias, const MlpNorm &norm, const double *x,
-                  const double *y, const double *z, int pairs, const unsigned int *list,
+                  const double *y, const double *z, int pairs, int stride, const unsigned int *list,
                   const unsigned long long *list_count, int n_host, int n_cap, GridDims g, int *guess, int num_sms,
-                  unsigned int *err, cudaStream_t s, float *yout, int stall_test) {
+                  unsigned int *err, cudaStream_t s, long long *cell3, float *yout, int stall_test) {
   static int attr_device = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -357,11 +360,11 @@ void mlp_guess_tc(const unsigned char *img, int bf16, const float *bias, const M
   if (blocks < 1) blocks = 1;
   const unsigned long long limit = stall_test ? 1024ull : WAIT_LIMIT;
   if (bf16)
-    k_mlp_guess_tc<true><<<(unsigned)blocks, TC_THREADS, SM_TOTAL, s>>>(img, bias, norm, x, y, z, pairs, list,
-                                                                        list_count, n_host, g, guess, yout, err,
+    k_mlp_guess_tc<true><<<(unsigned)blocks, TC_THREADS, SM_TOTAL, s>>>(img, bias, norm, x, y, z, pairs, stride, list,
+                                                                        list_count, n_host, g, guess, cell3, yout, err,
                                                                         limit, stall_test);
   else
-    k_mlp_guess_tc<false><<<(unsigned)blocks, TC_THREADS, SM_TOTAL, s>>>(img, bias, norm, x, y, z, pairs, list,
-                                                                         list_count, n_host, g, guess, yout, err,
+    k_mlp_guess_tc<false><<<(unsigned)blocks, TC_THREADS, SM_TOTAL, s>>>(img, bias, norm, x, y, z, pairs, stride, list,
+                                                                         list_count, n_host, g, guess, cell3, yout, err,
                                                                          limit, stall_test);
 }

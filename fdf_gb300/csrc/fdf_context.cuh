@@ -57,9 +57,11 @@ struct FdfContext {
   void *swarm_mem = nullptr;
   unsigned int *keys = nullptr, *perm = nullptr;   // [cap]: cell key per slot, sorted slot -> previous slot
   unsigned int *rank = nullptr;                    // [cap]: rank of the slot's particle within its new cell
-  unsigned int *cell_start = nullptr;              // [Nc+2]: histogram, then its exclusive scan
+  unsigned int *hist = nullptr;                    // [Nc+2]: cell histogram, zero between the runs
+  unsigned int *cell_start = nullptr;              // [Nc+2]: its exclusive scan
   unsigned int *scan_sums = nullptr;
   DevCounters *cnt = nullptr;
+  DevCounters *cnt_host = nullptr;                 // page-locked: DEVCOUNTERS_HEAD bytes of cnt
   void *staging = nullptr;
   size_t staging_bytes = 0;
   int xfer_route = FDF_TRANSFER_AUTO;     // fdf_SetTransferRoute
@@ -86,12 +88,14 @@ struct FdfContext {
   std::string c2c_msg;
   int c2c_flipped = 0;
   bool c2c_half = false;         // every tabled value mid-range: the halved Contra2Cart applies
-  // fdf_AdvanceSteps replays one captured step per swarm buffer parity; `gen` counts the
+  // the steps replay one captured step per swarm buffer parity; `gen` counts the
   // changes of anything a captured step bakes in (pointers, kernel arguments, form)
   long long gen = 1;
   cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
   long long graph_gen[2] = {0, 0};
-  long long eager_gen = 0;   // generation of the last eager step
+  long long graph_launches = 0;   // kernels of a captured step
+  long long eager_gen = 0;        // generation of the last eager step
+  int eager_steps = 0;            // eager steps since the generation changed (up to where it captures)
 };
 
 

@@ -86,3 +86,41 @@ __device__ __forceinline__ void block_add_u64(unsigned long long v, unsigned lon
     if (t) atomicAdd(dst, t);
   }
 }
+
+// The flush rows summed into the run's counters, and cleared.  One block of 256 threads (each two
+// rows); integer sums, so the totals do not depend on the flush order.
+__device__ __forceinline__ void fold_counts(DevCounters *cnt) {
+  static_assert(FDF_CNT_STRIPES == 512 && CNT_FB == 5, "two rows per thread, six slots each");
+  __shared__ unsigned long long part[8][6];
+  unsigned long long t[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    ulonglong2 *row = reinterpret_cast<ulonglong2 *>(cnt->stripes[threadIdx.x + 256 * h]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const ulonglong2 v = row[q];
+      t[2 * q] += v.x;
+      t[2 * q + 1] += v.y;
+      row[q] = make_ulonglong2(0ull, 0ull);
+    }
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    t[q] = warp_sum_u64(t[q]);
+    if (lane == 0) part[w][q] = t[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    unsigned long long v = 0;
+    for (int k = 0; k < 8; ++k) v += part[k][threadIdx.x];
+    switch (threadIdx.x) {
+      case CNT_LOST: cnt->removed_lost = v; break;
+      case CNT_OOB: cnt->removed_oob = v; break;
+      case CNT_EVALS: cnt->evals = v; break;
+      case CNT_EVALS_TOTAL: cnt->evals_total += v; break;
+      case CNT_LOST_TOTAL: cnt->lost_total = v; break;
+      default: cnt->fallbacks = v; cnt->fallbacks_total += v; break;
+    }
+  }
+}

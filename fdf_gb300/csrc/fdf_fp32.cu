@@ -158,7 +158,10 @@ __global__ void __launch_bounds__(FDF_LOC_THREADS, FDF_LOC_MIN_BLOCKS) k_locate3
                                                   unsigned int *__restrict__ pending, int n_cap, float far_cells) {
   const int n = cnt->n_sorted;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0 && advect) atomicAdd(&cnt->psteps_total, (unsigned long long)n);
+  if (s == 0) {
+    cnt->n_start = n;
+    if (advect) atomicAdd(&cnt->psteps_total, (unsigned long long)n);
+  }
   LocCounts m;
   unsigned int hkey = 0xffffffffu;
   bool wait = false;

@@ -37,15 +37,15 @@ enum { ST_NEEDS_LOCATION = 0, ST_ACTIVE_AND_LOCATED = 1, ST_MIGRATING_OUT = 2, S
 enum { ERRBIT_DEGENERATE = 1u, ERRBIT_TC_TIMEOUT = 4u };
 
 // The walk kernels' block flushes go to one of FDF_CNT_STRIPES rows (by block index), so that
-// they spread over the L2 slices instead of queueing on one line; k_fold_counts adds the rows
-// to the counters at the end of every pipeline run and zeroes them.
+// they spread over the L2 slices instead of queueing on one line; the slot scatter's last block
+// (fold_counts) sums the rows into the counters of every pipeline run and zeroes them.
 #define FDF_CNT_STRIPES 512
 enum { CNT_LOST = 0, CNT_OOB = 1, CNT_EVALS = 2, CNT_EVALS_TOTAL = 3, CNT_LOST_TOTAL = 4, CNT_FB = 5,
        CNT_SLOTS = 8 };
 
 // Counters kept on the device so that a step needs no host round trip.
 struct DevCounters {
-  // reset at the start of every pipeline run
+  // of the last pipeline run
   unsigned long long removed_lost;
   unsigned long long removed_oob;
   unsigned long long evals;        // walk evaluations the reference makes for this run (cycles count MAX_TRAVERSAL)
@@ -54,7 +54,7 @@ struct DevCounters {
   unsigned long long pending;      // learned form: particles that left their previous cell
   // kept across runs
   unsigned int err;
-  unsigned int pad;
+  int n_start;      // particles held at the start of the last pipeline run
   int n;            // live particle count after the last removal
   int n_sorted;     // particles held in the arrays (live + LOST kept by the initial setup)
   unsigned long long psteps_total;  // sum over steps of the particles at step start (never reset per step)
@@ -65,7 +65,8 @@ struct DevCounters {
   unsigned long long guess_taken_total;   // ... their walks' evaluations after P1 whose cell lay on the guessed path
   unsigned long long guess_evals_total;   // ... evaluations made by their walks from P1
   unsigned long long fallback_evals_total;   // (unused: zero)
-  unsigned long long stripes[FDF_CNT_STRIPES][CNT_SLOTS];   // pending block flushes (k_fold_counts)
+  // pending block flushes (fold_counts); rows of 64 bytes
+  alignas(64) unsigned long long stripes[FDF_CNT_STRIPES][CNT_SLOTS];
 };
 // The counters without the flush rows (what the host reads back).
 #define DEVCOUNTERS_HEAD offsetof(DevCounters, stripes)
@@ -170,8 +171,6 @@ void launch_move_kept(const SwarmBuf &src, const SwarmBuf &dst, int a, int b, in
 // The plain form's k-faces of layer k summed again from seeds (fdf_DepositKFaceLayer).
 void launch_deposit_k_layer(const SwarmBuf &b, GridDims g, const unsigned int *cell_start, int k, double volume,
                             const double *seed, const double *seed_mom, double *fk, double *mk, cudaStream_t s);
-// Adds the pending block flushes to the counters and clears them (end of a pipeline run).
-void launch_fold_counts(DevCounters *cnt, cudaStream_t s);
 void launch_build_planes(const double *coor_aos, GridDims g, double *planes, unsigned int *err, cudaStream_t s);
 // cell_start == nullptr: every node; else only nodes adjacent to an occupied cell.
 void launch_center_to_corner(const double *ucat, GridDims g, double *corner, const unsigned int *cell_start,
@@ -208,10 +207,13 @@ void launch_deposit(const SwarmBuf &b, GridDims g, const unsigned int *cell_star
 // Counting sort helpers (fdf_sort.cu).
 size_t scan_scratch_words(long long count);
 long long scan_max_count();
-void exclusive_scan_u32(unsigned int *data, long long count, unsigned int *sums, cudaStream_t s);
+// In-place exclusive scan, and the cell histogram's into cell_start, which leaves the histogram zero
+// for the next run.  Both return the kernels launched.
+int exclusive_scan_u32(unsigned int *data, long long count, unsigned int *sums, cudaStream_t s);
+int scan_histogram(unsigned int *hist, unsigned int *cell_start, long long count, unsigned int *sums, cudaStream_t s);
 // perm[cell_start[key] + rank[s]] = s for every kept particle (keys and ranks from the locate
-// kernels' histogram).
-void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, int n_cap, const DevCounters *cnt,
+// kernels' histogram); folds the walk's counters.
+void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, int n_cap, DevCounters *cnt,
                           unsigned int sentinel, int keep_lost, const unsigned int *cell_start, unsigned int *perm,
                           cudaStream_t s);
 // Orders every cell's slots by (PID, previous slot), or by previous slot when pid is null; with

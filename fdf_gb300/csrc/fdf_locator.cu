@@ -293,7 +293,7 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
                   ctx->sentinel, s);
   mlp_flag_located(tb.cell, tb.status, n, flag, s);
   CUT(cudaMemcpyAsync(slot, flag, 4ull * n, cudaMemcpyDeviceToDevice, s));
-  exclusive_scan_u32(slot, n, sums, s);
+  ctx->launches += exclusive_scan_u32(slot, n, sums, s);
   CUT(cudaGetLastError());
   unsigned int last[2] = {0, 0};
   CUT(cudaMemcpyAsync(&last[0], slot + n - 1, 4, cudaMemcpyDeviceToHost, s));
@@ -313,7 +313,7 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   CUT(cudaMalloc((void **)&xs, 12ull * m));
   CUT(cudaMalloc((void **)&ts, 12ull * m));
   mlp_make_samples(tb.x, tb.y, tb.z, tb.cell, slot, flag, n, L.norm, g, xs, ts, s);
-  ctx->launches += 4 + 3;
+  ctx->launches += 4;
   // --- training
   const int B = (int)batch;
   int r = ensure_scratch(ctx, B);

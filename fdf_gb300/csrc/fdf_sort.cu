@@ -15,6 +15,7 @@
 //      previous slot alone (a stable counting sort: the same on every run for the same
 //      input, and no gather of the PIDs), as does the standalone sort.
 #include "fdf_internal.cuh"
+#include "fdf_counters.cuh"
 
 #include <algorithm>
 
@@ -92,24 +93,43 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(unsigned int *sums, 
   }
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(unsigned int *__restrict__ data, long long count,
-                                                            const unsigned int *__restrict__ sums) {
+// out = exclusive scan of in (out == in allowed).  DIRECT: sums holds the blocks' own sums and each
+// block adds up those before it, which spares the launch that scans them; clear: `in` is left zero
+// (the histogram of the next step).
+template <bool DIRECT>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(unsigned int *in, unsigned int *out, long long count,
+                                                            const unsigned int *__restrict__ sums, int clear) {
   long long base = (long long)blockIdx.x * SCAN_BLOCK + (long long)threadIdx.x * SCAN_ITEMS;
   unsigned int v[SCAN_ITEMS], t = 0;
-  load8(data, base, count, v);
+  load8(in, base, count, v);
+  unsigned int before;
+  if (DIRECT) {
+    unsigned int part = 0;
+    for (int q = threadIdx.x; q < (int)blockIdx.x; q += SCAN_THREADS) part += sums[q];
+    block_exclusive_scan(part, &before);
+  } else {
+    before = sums[blockIdx.x];
+  }
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) t += v[q];
-  unsigned int ex = block_exclusive_scan(t, nullptr) + sums[blockIdx.x];
+  unsigned int ex = block_exclusive_scan(t, nullptr) + before;
   unsigned int o[SCAN_ITEMS];
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) { o[q] = ex; ex += v[q]; }
-  if (base + SCAN_ITEMS <= count && ((reinterpret_cast<size_t>(data + base) & 15) == 0)) {
-    *reinterpret_cast<uint4 *>(data + base) = make_uint4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<uint4 *>(data + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+  if (base + SCAN_ITEMS <= count && ((reinterpret_cast<size_t>(in + base) | reinterpret_cast<size_t>(out + base)) & 15) == 0) {
+    *reinterpret_cast<uint4 *>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4 *>(out + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+    if (clear) {
+      *reinterpret_cast<uint4 *>(in + base) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4 *>(in + base + 4) = make_uint4(0u, 0u, 0u, 0u);
+    }
   } else {
 #pragma unroll
     for (int q = 0; q < SCAN_ITEMS; ++q)
-      if (base + q < count) data[base + q] = o[q];
+      if (base + q < count) {
+        out[base + q] = o[q];
+        if (clear) in[base + q] = 0u;
+      }
   }
 }
 
@@ -122,11 +142,17 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(unsigned int *__res
 #ifndef FDF_SCATTER_ITEMS
 #define FDF_SCATTER_ITEMS 4
 #endif
+// The last block folds the counters' flush rows instead (the walk has ended): a launch of its own
+// took 13 us at the end of every step, this runs beside the slots.
 __global__ void __launch_bounds__(256) k_scatter_slots(const unsigned int *__restrict__ keys,
-                                                      const unsigned int *__restrict__ rank, const DevCounters *cnt,
+                                                      const unsigned int *__restrict__ rank, DevCounters *cnt,
                                                       unsigned int sentinel, int keep_lost,
                                                       const unsigned int *__restrict__ cell_start,
                                                       unsigned int *__restrict__ perm) {
+  if (blockIdx.x == gridDim.x - 1) {
+    fold_counts(cnt);
+    return;
+  }
   constexpr int IT = FDF_SCATTER_ITEMS;
   const long long n = cnt->n_sorted;
   const long long base = (long long)blockIdx.x * IT * blockDim.x + threadIdx.x;
@@ -489,21 +515,37 @@ size_t scan_scratch_words(long long count) { return (size_t)((count + SCAN_BLOCK
 
 long long scan_max_count() { return (long long)SCAN_BLOCK * SCAN_THREADS * SUMS_PER_THREAD; }
 
-void exclusive_scan_u32(unsigned int *data, long long count, unsigned int *sums, cudaStream_t s) {
-  long long blocks = (count + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  if (blocks < 1) blocks = 1;
-  k_scan_reduce<<<(unsigned)blocks, SCAN_THREADS, 0, s>>>(data, count, sums);
+// Blocks of a scan whose offsets each block adds up itself: up to here (33M values) the launch saved
+// (2.5 us) outweighs the sums read again, half the blocks' count by each (14M cells: 3 MB in all).
+constexpr long long SCAN_DIRECT = 4096;
+
+static int exclusive_scan(unsigned int *in, unsigned int *out, long long count, unsigned int *sums, int clear,
+                          cudaStream_t s) {
+  const long long blocks = std::max<long long>((count + SCAN_BLOCK - 1) / SCAN_BLOCK, 1);
+  k_scan_reduce<<<(unsigned)blocks, SCAN_THREADS, 0, s>>>(in, count, sums);
+  if (blocks <= SCAN_DIRECT) {
+    k_scan_apply<true><<<(unsigned)blocks, SCAN_THREADS, 0, s>>>(in, out, count, sums, clear);
+    return 2;
+  }
   k_scan_sums<<<1, SCAN_THREADS, 0, s>>>(sums, (int)blocks);
-  k_scan_apply<<<(unsigned)blocks, SCAN_THREADS, 0, s>>>(data, count, sums);
+  k_scan_apply<false><<<(unsigned)blocks, SCAN_THREADS, 0, s>>>(in, out, count, sums, clear);
+  return 3;
 }
 
-void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, int n_cap, const DevCounters *cnt,
+int exclusive_scan_u32(unsigned int *data, long long count, unsigned int *sums, cudaStream_t s) {
+  return exclusive_scan(data, data, count, sums, 0, s);
+}
+
+int scan_histogram(unsigned int *hist, unsigned int *cell_start, long long count, unsigned int *sums, cudaStream_t s) {
+  return exclusive_scan(hist, cell_start, count, sums, 1, s);
+}
+
+void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, int n_cap, DevCounters *cnt,
                           unsigned int sentinel, int keep_lost, const unsigned int *cell_start, unsigned int *perm,
                           cudaStream_t s) {
   const int th = 256, per_block = th * FDF_SCATTER_ITEMS;
   int blocks = (n_cap + per_block - 1) / per_block;
-  if (blocks == 0) blocks = 1;
-  k_scatter_slots<<<blocks, th, 0, s>>>(keys, rank, cnt, sentinel, keep_lost, cell_start, perm);
+  k_scatter_slots<<<blocks + 1, th, 0, s>>>(keys, rank, cnt, sentinel, keep_lost, cell_start, perm);
 }
 
 int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,

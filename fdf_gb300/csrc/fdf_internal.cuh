@@ -221,7 +221,8 @@ void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, in
 int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
                            unsigned int *lost_scratch, int n_cap, cudaStream_t s);
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
-                          unsigned int *cell_start, unsigned int *cursor, unsigned int *sums, cudaStream_t s);
+                          unsigned int *cell_start, unsigned int *rank, unsigned int *cursor, unsigned int *sums,
+                          cudaStream_t s);
 
 // AoS <-> SoA marshalling of the DMSwarm fields.
 void launch_swarm_from_aos(const double *pos, const double *vel, const double *wgt, const double *P,

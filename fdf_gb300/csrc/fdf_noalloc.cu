@@ -73,6 +73,6 @@ extern "C" int fdf_SortByCellNoAlloc(const int32_t *cell_ids, int64_t n, int64_t
   if (r) return r;
   unsigned int *cursor = scratch;
   unsigned int *sums = scratch + NOALLOC_CURSOR_WORDS;
-  cell_sort_on_scratch(cell_ids, n, ncells, perm, cell_start, cursor, sums, (cudaStream_t)stream);
+  cell_sort_on_scratch(cell_ids, n, ncells, perm, cell_start, nullptr, cursor, sums, (cudaStream_t)stream);
   return cudaGetLastError() == cudaSuccess ? FDF_SUCCESS : FDF_ERR_GPU;
 }

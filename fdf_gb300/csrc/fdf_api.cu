@@ -724,7 +724,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
                      m, m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, s);
   } else {
     double *m = ctx->momentum ? ctx->mom : nullptr;
-    launch_deposit(dst, g, ctx->cell_start, ctx->volume, ctx->count, ctx->avg, ctx->fi, ctx->fj, ctx->fk, m,
+    launch_deposit(dst, ctx->cap, g, ctx->cell_start, ctx->volume, ctx->count, ctx->avg, ctx->fi, ctx->fj, ctx->fk, m,
                    m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, s);
   }
   ctx->out_momentum = ctx->momentum;
@@ -866,7 +866,7 @@ int fdf_ScatterAllParticleFieldsToEulerFields(FdfContext *ctx) {
                      m, m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, ctx->stream);
   } else {
     double *m = ctx->momentum ? ctx->mom : nullptr;
-    launch_deposit(b, g, ctx->cell_start, ctx->volume, ctx->count, ctx->avg, ctx->fi, ctx->fj, ctx->fk, m,
+    launch_deposit(b, ctx->cap, g, ctx->cell_start, ctx->volume, ctx->count, ctx->avg, ctx->fi, ctx->fj, ctx->fk, m,
                    m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, ctx->stream);
   }
   CHECK_LAUNCH();

@@ -200,7 +200,7 @@ void launch_gather_interp(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, G
                           const double *corner, const unsigned int *perm, const unsigned int *cell_start,
                           DevCounters *cnt, cudaStream_t s, int mode = GATHER_INTERP);
 // mi, mj, mk (SoA [3][faces], or nullptr): the momentum deposit, V * velocity split like the volume.
-void launch_deposit(const SwarmBuf &b, GridDims g, const unsigned int *cell_start, double volume, double *count,
+void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, double *count,
                     double *avg, double *fi, double *fj, double *fk, double *mi, double *mj, double *mk,
                     cudaStream_t s);
 

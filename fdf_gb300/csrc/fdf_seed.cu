@@ -17,55 +17,63 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   return z ^ (z >> 31);
 }
 
-// uniform01(seed, stream)[idx] of workloads.py
+// uniform01(seed, stream)[idx] of workloads.py: the top 53 bits of the stream's word, times 2^-53.
+// Exact, so it is put together from the bits.
 __device__ __forceinline__ double uniform01(unsigned long long seed, unsigned long long stream,
                                             unsigned long long idx) {
   const unsigned long long base =
       mix64(seed * 0xD1B54A32D192ED03ULL + stream * 0xA24BAED4963EE407ULL + 0x632BE59BD9B4E019ULL);
-  const unsigned long long z = mix64(base + (idx + 1ULL) * 0x9E3779B97F4A7C15ULL);
-  return (double)(z >> 11) * (1.0 / 9007199254740992.0);
+  const unsigned long long k = mix64(base + (idx + 1ULL) * 0x9E3779B97F4A7C15ULL) >> 11;
+  if (k == 0ull) return 0.0;
+  const int lz = __clzll((long long)k);   // 11 .. 63
+  return __longlong_as_double((long long)(((unsigned long long)(1032 - lz) << 52) + (k << (lz - 11))));
 }
 
-__global__ void k_seed(const double *__restrict__ coor, GridDims g, long long n, unsigned long long seed,
-                       long long pid_base, int hint, int form32, double P0, SwarmBuf b) {
+// (long long)x for 0 <= x < 2^31.
+__device__ __forceinline__ int truncate(double x) {
+  const unsigned long long u = fdfx::ubits(x);
+  const int e = (int)(u >> 52) - 1023;
+  return e < 0 ? 0 : (int)(((u & 0x000fffffffffffffull) | 0x0010000000000000ull) >> (52 - e));
+}
+
+// Bound by FP64 when written with it (118 FP64 instructions per particle, 12.0 ms for 64M of them in
+// 14M cells): the conversions, the clamps and the 39 products run on the integer pipe, with the same
+// bits, and 24 subtractions and additions are left: 9.5 ms, by the random gathers of eight nodes.
+__global__ void k_seed(const double *__restrict__ coor, GridDims g, double dIM, double dJM, double dKM, long long n,
+                       unsigned long long seed, long long pid_base, int hint, int form32, double P0, float P0f,
+                       SwarmBuf b) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= n) return;
   const unsigned long long idx = (unsigned long long)p;
-  const double ri = uniform01(seed, 0, idx), rj = uniform01(seed, 1, idx), rk = uniform01(seed, 2, idx);
-  long long ci = (long long)fdfx::mul(ri, (double)g.IM), cj = (long long)fdfx::mul(rj, (double)g.JM),
-            ck = (long long)fdfx::mul(rk, (double)g.KM);
-  ci = ci < 0 ? 0 : (ci > g.IM - 1 ? g.IM - 1 : ci);
-  cj = cj < 0 ? 0 : (cj > g.JM - 1 ? g.JM - 1 : cj);
-  ck = ck < 0 ? 0 : (ck > g.KM - 1 ? g.KM - 1 : ck);
+  const double r[3] = {uniform01(seed, 0, idx), uniform01(seed, 1, idx), uniform01(seed, 2, idx)};
+  const int ci = min(truncate(fdfx::mul_int(r[0], dIM)), g.IM - 1), cj = min(truncate(fdfx::mul_int(r[1], dJM)), g.JM - 1),
+            ck = min(truncate(fdfx::mul_int(r[2], dKM)), g.KM - 1);
   const double lim = 1.0 - 1.0e-7;
-  double xi = uniform01(seed, 3, idx), eta = uniform01(seed, 4, idx), zta = uniform01(seed, 5, idx);
-  xi = fdfx::pmax(fdfx::pmin(xi, lim), 0.0);     // np.maximum(np.minimum(u, lim), 0.0) on [0,1) values
-  eta = fdfx::pmax(fdfx::pmin(eta, lim), 0.0);
-  zta = fdfx::pmax(fdfx::pmin(zta, lim), 0.0);
+  double t[3][2];   // the two weights of each direction: 1 - xi, xi
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {   // np.maximum(np.minimum(u, lim), 0.0) on [0,1) values, ordered as their bits are
+    const unsigned long long u = min(fdfx::ubits(uniform01(seed, 3 + d, idx)), fdfx::ubits(lim));
+    t[d][1] = __longlong_as_double((long long)u);
+    t[d][0] = fdfx::sub(1.0, t[d][1]);
+  }
   double x = 0.0, y = 0.0, z = 0.0;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    const double a = (c & 1) ? xi : fdfx::sub(1.0, xi);
-    const double bb = (c & 2) ? eta : fdfx::sub(1.0, eta);
-    const double cc = (c & 4) ? zta : fdfx::sub(1.0, zta);
-    const double N = fdfx::mul(fdfx::mul(a, bb), cc);
-    const long long ii = ci + ((c & 1) ? 1 : 0), jj = cj + ((c & 2) ? 1 : 0), kk = ck + ((c & 4) ? 1 : 0);
+    const double N = fdfx::mul_int(fdfx::mul_int(t[0][c & 1], t[1][(c >> 1) & 1]), t[2][c >> 2]);
+    const long long ii = ci + (c & 1), jj = cj + ((c >> 1) & 1), kk = ck + (c >> 2);
     const double *V = coor + 3 * ((kk * (g.JM + 1) + jj) * (long long)(g.IM + 1) + ii);
-    x = fdfx::add(x, fdfx::mul(N, V[0]));
-    y = fdfx::add(y, fdfx::mul(N, V[1]));
-    z = fdfx::add(z, fdfx::mul(N, V[2]));
+    const double vx = fdfx::mul_int(N, V[0]), vy = fdfx::mul_int(N, V[1]), vz = fdfx::mul_int(N, V[2]);
+    x = c ? fdfx::add(x, vx) : fdfx::add0(vx);
+    y = c ? fdfx::add(y, vy) : fdfx::add0(vy);
+    z = c ? fdfx::add(z, vz) : fdfx::add0(vz);
   }
   if (form32) {
     const double v[3] = {x, y, z};
     double *dst[3] = {b.x, b.y, b.z};
-    for (int q = 0; q < 3; ++q) {
-      const float h = __double2float_rn(v[q]);
-      const float l = __double2float_rn(__dsub_rn(v[q], (double)h));
-      *reinterpret_cast<float2 *>(dst[q] + p) = make_float2(h, l);
-    }
+    for (int q = 0; q < 3; ++q) *reinterpret_cast<float2 *>(dst[q] + p) = fdfx::split_rn(v[q]);
     b.uf[p] = 0.f; b.vf[p] = 0.f; b.wf[p] = 0.f;
     b.a1f[p] = 0.f; b.a2f[p] = 0.f; b.a3f[p] = 0.f;
-    b.Pf[p] = (float)P0;
+    b.Pf[p] = P0f;
   } else {
     b.x[p] = x; b.y[p] = y; b.z[p] = z;
     b.u[p] = 0.0; b.v[p] = 0.0; b.w[p] = 0.0;
@@ -73,7 +81,7 @@ __global__ void k_seed(const double *__restrict__ coor, GridDims g, long long n,
     b.P[p] = P0;
   }
   b.pid[p] = pid_base + p;
-  b.cell[p] = hint ? (int)((ck * g.JM + cj) * g.IM + ci) : -1;
+  b.cell[p] = hint ? (int)(((long long)ck * g.JM + cj) * g.IM + ci) : -1;
   b.status[p] = ST_UNINITIALIZED;
 }
 
@@ -82,5 +90,6 @@ __global__ void k_seed(const double *__restrict__ coor, GridDims g, long long n,
 void launch_seed(const double *coor, GridDims g, long long n, unsigned long long seed, long long pid_base, int hint,
                  int form32, double P0, const SwarmBuf &b, cudaStream_t s) {
   if (n <= 0) return;
-  k_seed<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(coor, g, n, seed, pid_base, hint, form32, P0, b);
+  k_seed<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(coor, g, (double)g.IM, (double)g.JM, (double)g.KM, n, seed,
+                                                    pid_base, hint, form32, P0, (float)P0, b);
 }

@@ -88,6 +88,7 @@ int fdf_ContextDestroy(FdfContext *ctx) {
   cfree(ctx->swarm_mem); cfree(ctx->keys); cfree(ctx->perm); cfree(ctx->rank);
   cfree(ctx->hist); cfree(ctx->cell_start); cfree(ctx->scan_sums); cfree(ctx->cnt); cfree(ctx->staging);
   if (ctx->cnt_host) cudaFreeHost(ctx->cnt_host);
+  work_release(ctx);
   locator_free(ctx);
   for (auto &gx : ctx->step_graph)
     if (gx) cudaGraphExecDestroy(gx);
@@ -120,6 +121,7 @@ int fdf_SetGrid(FdfContext *ctx, int64_t IM, int64_t JM, int64_t KM, const doubl
   ctx->layout_ok = false;
   ctx->loc.has_params = false;   // a locator is trained for one grid
   ctx->gen++;
+  work_release(ctx);
   cfree(ctx->coor); cfree(ctx->planes); cfree(ctx->ucat); cfree(ctx->corner);
   cfree(ctx->count); cfree(ctx->avg); cfree(ctx->fi); cfree(ctx->fj); cfree(ctx->fk); cfree(ctx->cell_start); cfree(ctx->hist);
   cfree(ctx->scan_sums);
@@ -269,6 +271,7 @@ int fdf_ReserveParticles(FdfContext *ctx, int64_t capacity) {
   ctx->buf[1] = SwarmBuf{};
   ctx->staging_bytes = 0;
   ctx->gen++;
+  work_release(ctx);
   cfree(ctx->swarm_mem); cfree(ctx->keys); cfree(ctx->perm); cfree(ctx->rank); cfree(ctx->staging);
   int cap = (int)(capacity < 256 ? 256 : capacity);   // never zero: the sort always has scratch
   size_t per = swarm_bytes_per_buf(cap);
@@ -889,51 +892,30 @@ int fdf_LocatePoints(FdfContext *ctx, int64_t n, const double *position, const i
   cudaStream_t s = ctx->stream;
   const GridDims &g = ctx->g;
   const int m = (int)n;
-  // the points as a temporary plain-form swarm: NEEDS_LOCATION, walk start = the given cell
-  void *mem = nullptr;
-  const size_t sw = swarm_bytes_per_buf(m), aos = 24ull * m, one = 8ull * m;
-  const size_t bytes = sw + 4 * aos + 3 * one + 4ull * m + 4ull * (g.Nc + 2) + sizeof(DevCounters) + 256 * 12;
-  CU(cudaMalloc(&mem, bytes));
-  char *p = (char *)mem;
-  SwarmBuf tb;
-  carve_swarm(p, m, tb);
-  auto take = [&](size_t nb) { char *q = p; p += (nb + 255) / 256 * 256; return q; };
-  take(sw);
-  double *d_pos = (double *)take(aos);
-  long long *d_cell = (long long *)take(aos);
-  double *d_zero = (double *)take(aos);   // velocity, weight, P, pid, status (0 = NEEDS_LOCATION)
-  double *d_w = (double *)take(aos);
-  double *d_P = (double *)take(one);
-  long long *d_pid = (long long *)take(one);
-  long long *d_st = (long long *)take(one);
-  unsigned int *keys = (unsigned int *)take(4ull * m);
-  unsigned int *hist = (unsigned int *)take(4ull * (g.Nc + 2));
-  DevCounters *tc = (DevCounters *)take(sizeof(DevCounters));
-  DevCounters c0{};
-  c0.n = m;
-  c0.n_sorted = m;
+  // positions [n][3], cells [n][3] in and out, weights [n][3], statuses [n], the error word and the
+  // walk's scratch rows
+  const size_t aos = 24ull * m, one = 8ull * m, counters = (sizeof(DevCounters) + 255) / 256 * 256;
+  CallBuffer buf;
+  CU(buf.take(ctx, counters + 3 * aos + one));
+  DevCounters *tc = (DevCounters *)buf.p;
+  double *d_pos = (double *)(buf.p + counters);
+  long long *d_cell = (long long *)(d_pos + 3ull * m);
+  double *d_w = (double *)(d_cell + 3ull * m);
+  long long *d_st = (long long *)(d_w + 3ull * m);
   cudaError_t e = cudaMemcpyAsync(d_pos, position, aos, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = cell_in ? cudaMemcpyAsync(d_cell, cell_in, aos, cudaMemcpyHostToDevice, s) : cudaMemsetAsync(d_cell, 0xff, aos, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_zero, 0, aos, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, 4ull * (g.Nc + 2), s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(tc, &c0, sizeof(c0), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess && cell_in) e = cudaMemcpyAsync(d_cell, cell_in, aos, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(&tc->err, 0, sizeof(tc->err), s);
   if (e == cudaSuccess) {
-    launch_swarm_from_aos(d_pos, d_zero, d_zero, d_zero, d_cell, (const long long *)d_zero, (const long long *)d_zero,
-                          m, g, tb, s);
-    launch_locate(tb, m, g, ctx->table32, ctx->planes, 0.0, 0, ctx->bbox, 0, tc, keys, nullptr, hist, ctx->sentinel,
-                    s);
-    launch_swarm_to_aos(tb, m, g, d_pos, d_zero, d_w, d_P, d_cell, d_pid, d_st, s);
-    ctx->launches += 3;
+    launch_locate_points(d_pos, cell_in ? d_cell : nullptr, m, g, ctx->table32, ctx->planes, tc, d_cell, d_w, d_st, s);
+    ctx->launches += 1;
     e = cudaGetLastError();
   }
-  unsigned int err = 0;
+  unsigned int &err = ctx->cnt_host->err;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&err, &tc->err, sizeof(err), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cell_out, d_cell, aos, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(weight, d_w, aos, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(status, d_st, one, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&err, &tc->err, sizeof(err), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(mem);
   if (e != cudaSuccess) return fail(ctx, FDF_ERR_GPU, std::string("fdf_LocatePoints: ") + cudaGetErrorString(e));
   if (err & ERRBIT_DEGENERATE) return fail(ctx, FDF_ERR_USER, "Degenerate plane detected (normal vector is near zero).");
   return FDF_SUCCESS;
@@ -950,45 +932,26 @@ int fdf_InterpolatePoints(FdfContext *ctx, int64_t n, const int64_t *cell, const
   cudaStream_t s = ctx->stream;
   const GridDims &g = ctx->g;
   const int m = (int)n;
-  // the points as a temporary plain-form swarm in their own order (no sort): cells and weights
-  // in, velocities out; cell_start only carries the count the gather reads at [Nc], [Nc + 1]
-  void *mem = nullptr;
-  const size_t sw = swarm_bytes_per_buf(m), aos = 24ull * m, one = 8ull * m;
-  const size_t bytes = sw + 4 * aos + 3 * one + 4ull * (g.Nc + 2) + sizeof(DevCounters) + 256 * 10;
-  CU(cudaMalloc(&mem, bytes));
-  char *p = (char *)mem;
-  SwarmBuf tb;
-  carve_swarm(p, m, tb);
-  auto take = [&](size_t nb) { char *q = p; p += (nb + 255) / 256 * 256; return q; };
-  take(sw);
-  double *d_w = (double *)take(aos);
-  long long *d_cell = (long long *)take(aos);
-  double *d_zero = (double *)take(aos);     // position, velocity, P, pid, status (0 = NEEDS_LOCATION)
-  double *d_vel = (double *)take(aos);
-  double *d_P = (double *)take(one);
-  long long *d_pid = (long long *)take(one);
-  long long *d_st = (long long *)take(one);
-  unsigned int *cs = (unsigned int *)take(4ull * (g.Nc + 2));
-  DevCounters *tc = (DevCounters *)take(sizeof(DevCounters));
-  const unsigned int counts[2] = {(unsigned int)m, (unsigned int)m};
+  // cells [n][3], weights [n][3], velocities [n][3]
+  const size_t aos = 24ull * m;
+  CallBuffer buf;
+  CU(buf.take(ctx, 3 * aos));
+  long long *d_cell = (long long *)buf.p;
+  double *d_w = (double *)(d_cell + 3ull * m), *d_vel = d_w + 3ull * m;
   cudaError_t e = cudaMemcpyAsync(d_w, weight, aos, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_cell, cell, aos, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_zero, 0, aos, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(cs + g.Nc, counts, sizeof(counts), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(tc, 0, sizeof(DevCounters), s);
+  // Both ways are bound by FP64 adds, 21 per corner: eight corners for each point, or every node once
+  // (200,000 points in 2.1M cells: the node field alone took 90 of the call's 430 us, which takes 260
+  // now; one point 261 -> 45 us, most of it the call's own allocation).
+  const bool direct = 8ll * m < g.Nn;
   if (e == cudaSuccess) {
-    // every node of the corner field (the swarm steps compute only the nodes they need)
-    launch_center_to_corner(ctx->ucat, g, ctx->corner, nullptr, nullptr, s);
-    launch_swarm_from_aos(d_zero, d_zero, d_w, d_zero, d_cell, (const long long *)d_zero, (const long long *)d_zero,
-                          m, g, tb, s);
-    launch_gather_interp(tb, tb, m, g, ctx->corner, nullptr, cs, tc, s, INTERP_KEEP);
-    launch_swarm_to_aos(tb, m, g, d_zero, d_vel, d_w, d_P, d_cell, d_pid, d_st, s);
-    ctx->launches += 4;
+    if (!direct) launch_center_to_corner(ctx->ucat, g, ctx->corner, nullptr, nullptr, s);
+    launch_interp_points(d_cell, d_w, m, g, direct ? ctx->ucat : ctx->corner, direct, d_vel, s);
+    ctx->launches += direct ? 1 : 2;
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(velocity, d_vel, aos, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(mem);
   if (e != cudaSuccess) return fail(ctx, FDF_ERR_GPU, std::string("fdf_InterpolatePoints: ") + cudaGetErrorString(e));
   return FDF_SUCCESS;
 }

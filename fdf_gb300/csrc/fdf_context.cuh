@@ -64,6 +64,8 @@ struct FdfContext {
   DevCounters *cnt_host = nullptr;                 // page-locked: DEVCOUNTERS_HEAD bytes of cnt
   void *staging = nullptr;
   size_t staging_bytes = 0;
+  void *work = nullptr;                   // CallBuffer's memory between calls
+  size_t work_bytes = 0;
   int xfer_route = FDF_TRANSFER_AUTO;     // fdf_SetTransferRoute
   int route_up = -1, route_down = -1;     // AUTO: the route measured faster per direction (-1: not yet)
   unsigned int sentinel = 0;
@@ -156,6 +158,37 @@ inline cudaError_t dev_alloc(T **p, size_t bytes) {
   return dev_alloc_hooked(reinterpret_cast<void **>(p), bytes);
 }
 
+
+// Device memory for the length of one call (points, predictions).  Up to WORK_MAX it stays with the
+// context for the next call (an allocation and its release cost 150 us), until fdf_SetGrid or
+// fdf_ReserveParticles need the room; a larger one is released at the call's end.
+struct CallBuffer {
+  static constexpr size_t WORK_MAX = size_t(256) << 20;
+  char *p = nullptr;
+  bool own = false;
+  cudaError_t take(FdfContext *ctx, size_t bytes) {
+    if (bytes <= ctx->work_bytes) {
+      p = (char *)ctx->work;
+      return cudaSuccess;
+    }
+    own = bytes > WORK_MAX;
+    if (own) return cudaMalloc((void **)&p, bytes);
+    cfree(ctx->work);
+    ctx->work_bytes = 0;
+    const cudaError_t e = cudaMalloc(&ctx->work, bytes);
+    if (e != cudaSuccess) return e;
+    ctx->work_bytes = bytes;
+    p = (char *)ctx->work;
+    return cudaSuccess;
+  }
+  ~CallBuffer() {
+    if (own) cudaFree(p);
+  }
+};
+inline void work_release(FdfContext *ctx) {
+  cfree(ctx->work);
+  ctx->work_bytes = 0;
+}
 
 // Bytes of one swarm buffer, a multiple of 256: the second buffer of the pair starts at this
 // offset, and its arrays keep the 256-B alignment of the first's (the deposit's bulk copies need

@@ -6,6 +6,7 @@
 // reference (compiled without FMA) rounds it.
 #include "fdf_internal.cuh"
 #include "fdf_exact.cuh"
+#include "fdf_corner.cuh"
 #include "fdf_counters.cuh"
 #include <cfloat>
 
@@ -87,14 +88,9 @@ __global__ void k_build_planes(const double *__restrict__ coor, GridDims g, doub
   (void)err;
 }
 
-// InterpolateFieldFromCenterToCorner_Vector_Petsc, interpolation.c:598-679.
-// Each node averages its valid adjacent cells in (dk, dj, di) order.  The count is
-// a product of per-direction counts of 1 or 2, i.e. 1, 2, 4 or 8, so sum/count is
-// exactly sum*(1/count): both are the correctly rounded value of the same real.
-// The running sum starts at 0.0; "0.0 + first" is the first value except that a
-// -0.0 becomes +0.0 (add0).  With cell_start non-null, nodes none of whose
-// adjacent cells holds a particle are skipped: the corner field is an
-// intermediate of the interpolation and only those nodes are ever read.
+// The corner field (fdf_corner.cuh), one thread per node.  With cell_start non-null, nodes none of
+// whose adjacent cells holds a particle are skipped: the corner field is an intermediate of the
+// interpolation and only those nodes are ever read.
 // AOS: the output is [Nn][3] instead of [3][Nn] (for the host).
 template <bool AOS>
 __global__ void k_center_to_corner(const double *__restrict__ ucat, GridDims g, double *__restrict__ corner,
@@ -122,37 +118,8 @@ __global__ void k_center_to_corner(const double *__restrict__ ucat, GridDims g, 
   if (!work) return;
   int i, j, k;
   node_ijk(g, (unsigned int)q, i, j, k);
-  const double *ux = ucat, *uy = ucat + g.Nc, *uz = ucat + 2 * g.Nc;
-  double sx = 0.0, sy = 0.0, sz = 0.0;
-  int count = 0;
-#pragma unroll
-  for (int dk = -1; dk <= 0; ++dk) {
-    long long ck = k + dk;
-    if (ck < 0 || ck >= g.KM) continue;
-#pragma unroll
-    for (int dj = -1; dj <= 0; ++dj) {
-      long long cj = j + dj;
-      if (cj < 0 || cj >= g.JM) continue;
-#pragma unroll
-      for (int di = -1; di <= 0; ++di) {
-        long long ci = i + di;
-        if (ci < 0 || ci >= g.IM) continue;
-        long long c = (ck * g.JM + cj) * g.IM + ci;
-        double vx = __ldg(ux + c), vy = __ldg(uy + c), vz = __ldg(uz + c);
-        if (count == 0) {
-          sx = fdfx::add0(vx); sy = fdfx::add0(vy); sz = fdfx::add0(vz);
-        } else {
-          sx = add(sx, vx); sy = add(sy, vy); sz = add(sz, vz);
-        }
-        ++count;
-      }
-    }
-  }
-  double ox = 0.0, oy = 0.0, oz = 0.0;
-  if (count > 0) {
-    const int sh = count == 1 ? 0 : count == 2 ? 1 : count == 4 ? 2 : 3;   // sum * 0.5^sh, exact
-    ox = fdfx::scale_down(sx, sh); oy = fdfx::scale_down(sy, sh); oz = fdfx::scale_down(sz, sh);
-  }
+  double ox, oy, oz;
+  fdfx::corner_value(ucat, g, i, j, k, ox, oy, oz);
   if (AOS) {
     corner[3 * q] = ox; corner[3 * q + 1] = oy; corner[3 * q + 2] = oz;
   } else {

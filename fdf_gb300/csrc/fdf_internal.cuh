@@ -190,6 +190,14 @@ void launch_vec3_out(const float *soa, long long n, double *aos, cudaStream_t s)
 void launch_locate(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes, double dt,
                    int advect, const double *bbox, int drop_removed, DevCounters *cnt, unsigned int *keys,
                    unsigned int *rank, unsigned int *count, unsigned int sentinel, cudaStream_t s);
+// Points that are not the swarm, in the callers' [n][3] layout: their walk (cell_in may be null or
+// cell_out; cnt: its error word is set, its flush rows are scratch) and the velocity at their cells and
+// weights, from the corner field, or (direct) from ucat.
+void launch_locate_points(const double *pos, const long long *cell_in, int n, GridDims g, const float *table,
+                          const double *planes, DevCounters *cnt, long long *cell_out, double *weight, long long *status,
+                          cudaStream_t s);
+void launch_interp_points(const long long *cell, const double *weight, int n, GridDims g, const double *field, bool direct,
+                          double *vel, cudaStream_t s);
 // Modes of the gather kernels: sorted slot s takes the particle perm[s] (perm == nullptr: s
 // itself, src == dst allowed) for s < n = cell_start[Nc+1] (read on the device), and
 //   GATHER_INTERP  interpolates its velocity and sets its status from its cell (the step),

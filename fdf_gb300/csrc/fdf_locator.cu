@@ -255,19 +255,27 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   cudaStream_t s = ctx->stream;
   const GridDims &g = ctx->g;
   const long long n = n_samples;
-  // --- location pairs from the walking search
-  void *tmp_swarm = nullptr;
-  CU(cudaMalloc(&tmp_swarm, swarm_bytes_per_buf((int)n)));
-  SwarmBuf tb;
-  carve_swarm((char *)tmp_swarm, (int)n, tb);
-  DevCounters *tc = nullptr;
-  unsigned int *keys = nullptr, *hist = nullptr, *flag = nullptr, *slot = nullptr, *sums = nullptr;
-  float *xs = nullptr, *ts = nullptr, *hist_loss = nullptr;
-  auto release = [&]() {
-    cudaStreamSynchronize(s);
-    cudaFree(tmp_swarm); cudaFree(tc); cudaFree(keys); cudaFree(hist); cudaFree(flag); cudaFree(slot);
-    cudaFree(sums); cudaFree(xs); cudaFree(ts); cudaFree(hist_loss);
+  // --- location pairs from the walking search (one buffer for the call)
+  size_t bytes = 0;
+  auto part = [&](size_t b) {
+    const size_t at = bytes;
+    bytes += (b + 255) / 256 * 256;
+    return at;
   };
+  const size_t o_swarm = part(swarm_bytes_per_buf((int)n)), o_tc = part(sizeof(DevCounters)), o_keys = part(4ull * n),
+               o_hist = part(4ull * (g.Nc + 2)), o_flag = part(4ull * n), o_slot = part(4ull * n),
+               o_sums = part(4ull * scan_scratch_words(n)), o_xs = part(12ull * n), o_ts = part(12ull * n),
+               o_loss = part(4ull * (steps > 0 ? steps : 1));
+  CallBuffer buf;
+  CU(buf.take(ctx, bytes));
+  SwarmBuf tb;
+  carve_swarm(buf.p + o_swarm, (int)n, tb);
+  DevCounters *tc = (DevCounters *)(buf.p + o_tc);
+  unsigned int *keys = (unsigned int *)(buf.p + o_keys), *hist = (unsigned int *)(buf.p + o_hist),
+               *flag = (unsigned int *)(buf.p + o_flag), *slot = (unsigned int *)(buf.p + o_slot),
+               *sums = (unsigned int *)(buf.p + o_sums);
+  float *xs = (float *)(buf.p + o_xs), *ts = (float *)(buf.p + o_ts), *hist_loss = (float *)(buf.p + o_loss);
+  auto release = [&]() { cudaStreamSynchronize(s); };
 #define CUT(call)                                                                    \
   do {                                                                               \
     cudaError_t e_ = (call);                                                         \
@@ -277,12 +285,6 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
                   std::string(#call) + ": " + cudaGetErrorString(e_));               \
     }                                                                                \
   } while (0)
-  CUT(cudaMalloc((void **)&tc, sizeof(DevCounters)));
-  CUT(cudaMalloc((void **)&keys, 4ull * n));
-  CUT(cudaMalloc((void **)&hist, 4ull * (g.Nc + 2)));
-  CUT(cudaMalloc((void **)&flag, 4ull * n));
-  CUT(cudaMalloc((void **)&slot, 4ull * n));
-  CUT(cudaMalloc((void **)&sums, 4ull * scan_scratch_words(n)));
   DevCounters c0{};
   c0.n = (int)n;
   c0.n_sorted = (int)n;
@@ -310,8 +312,6 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
     release();
     return fail(ctx, FDF_ERR_ARG_WRONG, "fdf_LocatorTrain: the walk located none of the sample points");
   }
-  CUT(cudaMalloc((void **)&xs, 12ull * m));
-  CUT(cudaMalloc((void **)&ts, 12ull * m));
   mlp_make_samples(tb.x, tb.y, tb.z, tb.cell, slot, flag, n, L.norm, g, xs, ts, s);
   ctx->launches += 4;
   // --- training
@@ -319,7 +319,6 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   int r = ensure_scratch(ctx, B);
   if (r) { release(); return r; }
   TrainScratch S = carve_scratch(L.scratch, L.batch_cap);
-  CUT(cudaMalloc((void **)&hist_loss, 4ull * (steps > 0 ? steps : 1)));
   CUT(cudaMemsetAsync(S.err, 0, 4, s));
   float sc[3];
   loss_scale(ctx, sc);
@@ -364,8 +363,9 @@ static int locator_predict(FdfContext *ctx, const double *position, int64_t n, i
   cudaStream_t s = ctx->stream;
   // one buffer: positions [n][3] f64, cells [n][3] i64, outputs [n][3] f32, the error word
   const size_t off_cell = 24ull * n, off_out = off_cell + 24ull * n, off_err = off_out + (12ull * n + 255) / 256 * 256;
-  char *mem = nullptr;
-  CU(cudaMalloc((void **)&mem, off_err + 256));
+  CallBuffer buf;
+  CU(buf.take(ctx, off_err + 256));
+  char *mem = buf.p;
   double *d_pos = (double *)mem;
   long long *d_cell = (long long *)(mem + off_cell);
   float *d_out = (float *)(mem + off_out);
@@ -387,7 +387,6 @@ static int locator_predict(FdfContext *ctx, const double *position, int64_t n, i
     if (e == cudaSuccess && outputs) e = cudaMemcpyAsync(outputs, d_out, 12ull * n, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
-  cudaFree(mem);
   if (e != cudaSuccess) return fail(ctx, FDF_ERR_GPU, std::string("fdf_LocatorPredict: ") + cudaGetErrorString(e));
   if (errw & ERRBIT_TC_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "fdf_LocatorPredict: tensor-core wait timed out");
   return FDF_SUCCESS;

@@ -3,12 +3,54 @@
 // device SoA marshalling.
 #include "fdf_internal.cuh"
 #include "fdf_exact.cuh"
+#include "fdf_corner.cuh"
 
 namespace {
 
 using fdfx::add;
 using fdfx::sub;
 using fdfx::mul;
+
+// ComputeTrilinearWeights (interpolation.c:839-864) and TrilinearInterpolation_Vector (:957-1042): the
+// velocity from the eight corner values value(c, x, y, z), c in bit order (i, j, k).
+template <typename Value>
+__device__ __forceinline__ void trilinear(double a1, double a2, double a3, Value value, double &ux, double &uy,
+                                          double &uz) {
+  a1 = fdfx::clamp01(a1);
+  a2 = fdfx::clamp01(a2);
+  a3 = fdfx::clamp01(a3);
+  const double oa1 = sub(1.0, a1), oa2 = sub(1.0, a2), oa3 = sub(1.0, a3);
+  // w[c] = (x*y)*z as the reference evaluates it; the four (x*y) pair products are shared
+  // The 36 products run on the integer pipe (fdfx::mul_int, the same bits as the FP64
+  // multiply) and the sums on the FP64 pipe, so both pipes work at once.  Moving products back to
+  // the FP64 pipe (3 to 12 of them) is no faster: 4.64 to 5.28 against 4.66 ms for 64M particles.
+  auto wmul = [](double x, double y) { return fdfx::mul_int(x, y); };
+  const double p00 = wmul(oa1, oa2), p10 = wmul(a1, oa2), p01 = wmul(oa1, a2), p11 = wmul(a1, a2);
+  double w[8];
+  w[0] = wmul(p00, oa3); w[1] = wmul(p10, oa3); w[2] = wmul(p01, oa3); w[3] = wmul(p11, oa3);
+  w[4] = wmul(p00, a3);  w[5] = wmul(p10, a3);  w[6] = wmul(p01, a3);  w[7] = wmul(p11, a3);
+  // accumulators start at 0.0: the first "0.0 + t" is t except that -0.0 becomes +0.0
+  double ax, ay, az, sw;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    double vx, vy, vz;
+    value(c, vx, vy, vz);
+    const double tx = wmul(w[c], vx), ty = wmul(w[c], vy), tz = wmul(w[c], vz);
+    ax = c ? add(ax, tx) : fdfx::add0(tx);
+    ay = c ? add(ay, ty) : fdfx::add0(ty);
+    az = c ? add(az, tz) : fdfx::add0(tz);
+    sw = c ? add(sw, w[c]) : fdfx::add0(w[c]);
+  }
+  // sumW > 1e-14 (false for NaN); x / 1.0 == x exactly, so the common sumW == 1 skips the divides
+  if (!fdfx::is_nan(sw) && !fdfx::le_pos(sw, fdfx::ubits(1.0e-14))) {
+    if (fdfx::ubits(sw) == 0x3ff0000000000000ULL) {
+      ux = ax; uy = ay; uz = az;
+    } else {
+      const fdfx::Divisor dsw = fdfx::make_divisor(sw);
+      ux = fdfx::div_by(ax, dsw); uy = fdfx::div_by(ay, dsw); uz = fdfx::div_by(az, dsw);
+    }
+  }
+}
 
 // Sorted slot s takes the particle from slot perm[s] of the previous order, then
 // interpolates ucat to it: ComputeTrilinearWeights (interpolation.c:839-864) and
@@ -52,47 +94,42 @@ __global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf
     dst.status[s] = mode == GATHER_INTERP ? (unsigned char)ST_ACTIVE_AND_LOCATED : st;
     int i, j, k;
     cell_ijk(g, (unsigned int)cell, i, j, k);
-    a1 = fdfx::clamp01(a1);
-    a2 = fdfx::clamp01(a2);
-    a3 = fdfx::clamp01(a3);
-    const double oa1 = sub(1.0, a1), oa2 = sub(1.0, a2), oa3 = sub(1.0, a3);
-    // w[c] = (x*y)*z as the reference evaluates it; the four (x*y) pair products are shared
-    // The 36 products run on the integer pipe (fdfx::mul_int, the same bits as the FP64
-    // multiply) and the sums on the FP64 pipe, so both pipes work at once.  Moving products back to
-    // the FP64 pipe (6 to 18 of them) is no faster: 2.76 to 2.99 against 2.78 ms for 32M particles.
-    auto wmul = [](double x, double y) { return fdfx::mul_int(x, y); };
-    const double p00 = wmul(oa1, oa2), p10 = wmul(a1, oa2), p01 = wmul(oa1, a2), p11 = wmul(a1, a2);
-    double w[8];
-    w[0] = wmul(p00, oa3); w[1] = wmul(p10, oa3); w[2] = wmul(p01, oa3); w[3] = wmul(p11, oa3);
-    w[4] = wmul(p00, a3);  w[5] = wmul(p10, a3);  w[6] = wmul(p01, a3);  w[7] = wmul(p11, a3);
     const long long mx = g.IM + 1, my = g.JM + 1;
-    const long long q0 = ((long long)k * my + j) * mx + i;
-    const long long off[8] = {0, 1, mx, mx + 1, mx * my, mx * my + 1, mx * my + mx, mx * my + mx + 1};
-    const double *cx = corner, *cy = corner + g.Nn, *cz = corner + 2 * g.Nn;
-    // accumulators start at 0.0: the first "0.0 + t" is t except that -0.0 becomes +0.0
-    double ax = fdfx::add0(wmul(w[0], __ldg(cx + q0)));
-    double ay = fdfx::add0(wmul(w[0], __ldg(cy + q0)));
-    double az = fdfx::add0(wmul(w[0], __ldg(cz + q0)));
-    double sw = fdfx::add0(w[0]);
-#pragma unroll
-    for (int c = 1; c < 8; ++c) {
-      const long long q = q0 + off[c];
-      ax = add(ax, wmul(w[c], __ldg(cx + q)));
-      ay = add(ay, wmul(w[c], __ldg(cy + q)));
-      az = add(az, wmul(w[c], __ldg(cz + q)));
-      sw = add(sw, w[c]);
-    }
-    // sumW > 1e-14 (false for NaN); x / 1.0 == x exactly, so the common sumW == 1 skips the divides
-    if (!fdfx::is_nan(sw) && !fdfx::le_pos(sw, fdfx::ubits(1.0e-14))) {
-      if (fdfx::ubits(sw) == 0x3ff0000000000000ULL) {
-        ux = ax; uy = ay; uz = az;
-      } else {
-        const fdfx::Divisor dsw = fdfx::make_divisor(sw);
-        ux = fdfx::div_by(ax, dsw); uy = fdfx::div_by(ay, dsw); uz = fdfx::div_by(az, dsw);
-      }
-    }
+    const double *at = corner + (((long long)k * my + j) * mx + i);
+    trilinear(a1, a2, a3, [&](int c, double &vx, double &vy, double &vz) {
+      const long long off = (c & 1) + ((c & 2) ? mx : 0) + ((c & 4) ? mx * my : 0);
+      vx = __ldg(at + off); vy = __ldg(at + g.Nn + off); vz = __ldg(at + 2 * g.Nn + off);
+    }, ux, uy, uz);
   }
   dst.u[s] = ux; dst.v[s] = uy; dst.w[s] = uz;
+}
+
+// InterpolateEulerFieldToSwarm for particles the caller holds (fdf_InterpolatePoints), in the callers'
+// layout.  DIRECT: each point averages its eight corners from ucat itself, node by node as the corner
+// field's kernel does, instead of reading the whole corner field made for it.
+template <bool DIRECT>
+__global__ void __launch_bounds__(128) k_interp_points(const long long *__restrict__ cell,
+                                                      const double *__restrict__ weight, int n, GridDims g,
+                                                      const double *__restrict__ field, double *__restrict__ vel) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const long long i = cell[3 * (size_t)p], j = cell[3 * (size_t)p + 1], k = cell[3 * (size_t)p + 2];
+  double ux = 0.0, uy = 0.0, uz = 0.0;
+  if (i >= 0 && i < g.IM && j >= 0 && j < g.JM && k >= 0 && k < g.KM) {
+    const long long mx = g.IM + 1, my = g.JM + 1;
+    trilinear(weight[3 * (size_t)p], weight[3 * (size_t)p + 1], weight[3 * (size_t)p + 2],
+              [&](int c, double &vx, double &vy, double &vz) {
+                const int ni = (int)i + (c & 1), nj = (int)j + ((c >> 1) & 1), nk = (int)k + (c >> 2);
+                if (DIRECT) {
+                  fdfx::corner_value(field, g, ni, nj, nk, vx, vy, vz);
+                } else {
+                  const double *at = field + (((long long)nk * my + nj) * mx + ni);
+                  vx = __ldg(at); vy = __ldg(at + g.Nn); vz = __ldg(at + 2 * g.Nn);
+                }
+              },
+              ux, uy, uz);
+  }
+  vel[3 * (size_t)p] = ux; vel[3 * (size_t)p + 1] = uy; vel[3 * (size_t)p + 2] = uz;
 }
 
 // One thread per grid node (i<=IM, j<=JM, k<=KM).  The node-sized outputs are the
@@ -386,6 +423,13 @@ void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int
   else if (n_cap <= 5 * g.Nc)
     k_deposit<false, true><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
   else k_deposit<false, false><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
+}
+
+void launch_interp_points(const long long *cell, const double *weight, int n, GridDims g, const double *field, bool direct,
+                          double *vel, cudaStream_t s) {
+  const unsigned int blocks = (unsigned int)((n + 127) / 128);
+  if (direct) k_interp_points<true><<<blocks, 128, 0, s>>>(cell, weight, n, g, field, vel);
+  else k_interp_points<false><<<blocks, 128, 0, s>>>(cell, weight, n, g, field, vel);
 }
 
 void launch_move_kept(const SwarmBuf &src, const SwarmBuf &dst, int a, int b, int c, int n, cudaStream_t s) {

@@ -42,6 +42,30 @@ using fdfx::add;
 using fdfx::sub;
 using fdfx::mul;
 
+// The pair a walk in FP64 positions takes for a coordinate: (hi, lo) within 2^-48 |v| of v; a nonzero
+// |v| below 2^-120 (where the split's error is absolute) gives a NaN pair, whose faces all take the
+// FP64 route.
+__device__ __forceinline__ float2 walk_pair(double v) {
+  const unsigned long long mag = fdfx::ubits(v) & fdfx::ABS_MASK;
+  if (mag < (903ull << 52) && mag != 0ull) return make_float2(__int_as_float(0x7fc00000), 0.f);
+  return fdfx::split_rn(v);
+}
+
+// UpdateParticleWeights (ParticleSwarm.c:1010-1047) from the concluding cell's FP64 distances.
+__device__ __forceinline__ void exact_weights(const double *__restrict__ row, double x, double y, double z, double &a1,
+                                              double &a2, double &a3) {
+  double d[6];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) d[f] = exact_face(row, f, x, y, z);
+  const unsigned long long tol_bits = fdfx::ubits(FDF_INTERP_DIST_TOL);
+#pragma unroll
+  for (int f = 0; f < 6; ++f)
+    if (fdfx::le_pos(d[f], tol_bits)) d[f] = FDF_INTERP_DIST_TOL;
+  a1 = fdfx::div_rn(d[F_LEFT], add(d[F_LEFT], d[F_RIGHT]));
+  a2 = fdfx::div_rn(d[F_BOTTOM], add(d[F_BOTTOM], d[F_TOP]));
+  a3 = fdfx::div_rn(d[F_BACK], add(d[F_FRONT], d[F_BACK]));
+}
+
 __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
     k_locate(SwarmBuf b, GridDims g, const float *__restrict__ table, const double *__restrict__ planes, double dt,
                int advect, int reset_first, const double *__restrict__ bbox, int drop_removed, DevCounters *cnt,
@@ -68,17 +92,11 @@ __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
     int cell = b.cell[s];
     bool lost = false;
     if (st != ST_ACTIVE_AND_LOCATED) {
-      // (hi, lo) within 2^-48 |v| of v; a nonzero |v| below 2^-120 (where the split's error is
-      // absolute) gives a NaN pair, whose faces all take the FP64 route
-      auto split = [](double v) {
-        const unsigned long long mag = fdfx::ubits(v) & fdfx::ABS_MASK;
-        if (mag < (903ull << 52) && mag != 0ull) return make_float2(__int_as_float(0x7fc00000), 0.f);
-        return fdfx::split_rn(v);
-      };
       Walk32 w;
       w.i = 0; w.j = 0; w.k = 0;   // InitializeTraversalParameters: previous cell, else (0,0,0)
       if (cell >= 0 && (long long)cell < g.Nc) cell_ijk(g, (unsigned int)cell, w.i, w.j, w.k);
-      walk_ref32<true, false, false, true>(table, planes, g, split(x), split(y), split(z), FDF_MAX_TRAVERSAL, w, cnt, x, y, z);
+      walk_ref32<true, false, false, true>(table, planes, g, walk_pair(x), walk_pair(y), walk_pair(z),
+                                            FDF_MAX_TRAVERSAL, w, cnt, x, y, z);
       if (w.degenerate) m.err |= ERRBIT_DEGENERATE;
       m.evals += (unsigned int)(w.cycle ? FDF_MAX_TRAVERSAL : w.steps);
       m.done += w.evaluated();
@@ -88,17 +106,9 @@ __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
         st = ST_LOST;
       } else {
         cell = (int)(((long long)w.k * g.JM + w.j) * g.IM + w.i);
-        const double *row = planes + (long long)cell * FDF_ROW;
-        double d[6];
-#pragma unroll
-        for (int f = 0; f < 6; ++f) d[f] = exact_face(row, f, x, y, z);
-        const unsigned long long tol_bits = fdfx::ubits(FDF_INTERP_DIST_TOL);
-#pragma unroll
-        for (int f = 0; f < 6; ++f)
-          if (fdfx::le_pos(d[f], tol_bits)) d[f] = FDF_INTERP_DIST_TOL;
-        b.a1[s] = fdfx::div_rn(d[F_LEFT], add(d[F_LEFT], d[F_RIGHT]));
-        b.a2[s] = fdfx::div_rn(d[F_BOTTOM], add(d[F_BOTTOM], d[F_TOP]));
-        b.a3[s] = fdfx::div_rn(d[F_BACK], add(d[F_FRONT], d[F_BACK]));
+        double a1, a2, a3;
+        exact_weights(planes + (long long)cell * FDF_ROW, x, y, z, a1, a2, a3);
+        b.a1[s] = a1; b.a2[s] = a2; b.a3[s] = a3;
         st = ST_ACTIVE_AND_LOCATED;
       }
       b.cell[s] = cell;
@@ -127,7 +137,46 @@ __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
   block_flush_counts(m, cnt);
 }
 
+// The walk and the weights of points that are not the swarm (fdf_LocatePoints), in the callers' layout:
+// no swarm buffers, sort keys or histogram.  cell_in == cell_out is allowed (null: from cell (0,0,0)).
+__global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
+    k_locate_points(const double *__restrict__ pos, const long long *cell_in, int n, GridDims g,
+                    const float *__restrict__ table, const double *__restrict__ planes, DevCounters *cnt,
+                    long long *cell_out, double *__restrict__ weight, long long *__restrict__ status) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const double x = pos[3 * (size_t)p], y = pos[3 * (size_t)p + 1], z = pos[3 * (size_t)p + 2];
+  Walk32 w;
+  w.i = 0; w.j = 0; w.k = 0;
+  if (cell_in) {
+    const long long i = cell_in[3 * (size_t)p], j = cell_in[3 * (size_t)p + 1], k = cell_in[3 * (size_t)p + 2];
+    if (i >= 0 && i < g.IM && j >= 0 && j < g.JM && k >= 0 && k < g.KM) { w.i = (int)i; w.j = (int)j; w.k = (int)k; }
+  }
+  walk_ref32<true, false, false, true>(table, planes, g, walk_pair(x), walk_pair(y), walk_pair(z), FDF_MAX_TRAVERSAL, w,
+                                      cnt, x, y, z);
+  if (w.degenerate) atomicOr(&cnt->err, (unsigned int)ERRBIT_DEGENERATE);
+  const bool lost = w.lost || !w.concluded;
+  double a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  if (!lost) {
+    const long long cell = ((long long)w.k * g.JM + w.j) * g.IM + w.i;
+    exact_weights(planes + cell * FDF_ROW, x, y, z, a1, a2, a3);
+  }
+  cell_out[3 * (size_t)p] = lost ? -1 : w.i;
+  cell_out[3 * (size_t)p + 1] = lost ? -1 : w.j;
+  cell_out[3 * (size_t)p + 2] = lost ? -1 : w.k;
+  weight[3 * (size_t)p] = a1; weight[3 * (size_t)p + 1] = a2; weight[3 * (size_t)p + 2] = a3;
+  status[p] = lost ? ST_LOST : ST_ACTIVE_AND_LOCATED;
+}
+
 }  // namespace
+
+void launch_locate_points(const double *pos, const long long *cell_in, int n, GridDims g, const float *table,
+                          const double *planes, DevCounters *cnt, long long *cell_out, double *weight, long long *status,
+                          cudaStream_t s) {
+  constexpr int th = FDF_PLAIN_THREADS;
+  k_locate_points<<<(unsigned int)((n + th - 1) / th), th, 0, s>>>(pos, cell_in, n, g, table, planes, cnt, cell_out,
+                                                                 weight, status);
+}
 
 void launch_locate(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes, double dt,
                    int advect, const double *bbox, int drop_removed, DevCounters *cnt, unsigned int *keys,

@@ -32,6 +32,27 @@ __device__ __forceinline__ float silu_grad(float z) {
   return s * (1.0f + z * (1.0f - s));
 }
 
+// Programmatic dependent launch: a kernel launched with launch_after may begin before the one ahead of
+// it on the stream has ended (once that one's blocks have all called let_next_start, or ended) and
+// calls await_previous before it touches anything the earlier kernels write.
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Params, typename... Args>
+void launch_after(void (*kernel)(Params...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t s,
+                  Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // errors through cudaGetLastError
+}
+
 // Polls of an mbarrier before a tensor-core wait is given up.
 constexpr unsigned long long GT_WAIT_LIMIT = 1ull << 22;
 
@@ -92,6 +113,12 @@ __global__ void k_pack_bias(const float *__restrict__ params, float *__restrict_
 // the lane quarter of w % 4) take accumulator columns 0-31, 32-63, 64-95 and 96-127.  The tile's gradient partials
 // (dW of its rows, bias sums, loss) go to part [tile][MLP_PART_STRIDE] in the parameter layout;
 // k_train_update adds them in tile order, so the result does not depend on scheduling.
+//
+// A step is a chain of dependent rounds on 64 of the SMs (a batch of 8192), so it is bound by latency.
+// Each epilogue has its 32 columns in flight at once (two rounds of 16 before), and both kernels of a
+// step are launched to follow the one ahead without the stream's gap: the samples are gathered and the
+// tensor memory allocated while the update before still runs.  500 steps of 8192 with their call:
+// 19.2 -> 15.3 ms.
 //
 // Tensor memory: C1 columns 0-127, C2 128-255, C3 256-383, working accumulator 384-511; the
 // dH of a layer lands in the columns of the C it no longer needs.  Every wait is bounded: past
@@ -168,14 +195,6 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
   volatile unsigned *tflag = reinterpret_cast<volatile unsigned *>(smem + TT_SM_BAR + 12);
   const unsigned bar = smem_u32(smem + TT_SM_BAR), sb = smem_u32(smem);
   float *prt = part + tile * MLP_PART_STRIDE;
-  {
-    const uint4 *src = reinterpret_cast<const uint4 *>(wimg);
-    uint4 *dst = reinterpret_cast<uint4 *>(smem);
-    for (int q = tid; q < MLP_IMG_BYTES / 16; q += TT_THREADS) dst[q] = src[q];
-    for (int q = tid; q < 387; q += TT_THREADS)
-      bias[q] = params[q < 128 ? MLP_OFF_B1 + q : q < 256 ? MLP_OFF_B2 + q - 128 : q < 384 ? MLP_OFF_B3 + q - 256
-                                                                                       : MLP_OFF_B4 + q - 384];
-  }
   float tgt[3] = {0.f, 0.f, 0.f};
   if (cg == 0) {   // the sample: X row [hi x, y, z, lo x, y, z, 0, ...], its target in registers
     float x[3] = {0.f, 0.f, 0.f};
@@ -210,6 +229,17 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
+  // up to here only the samples were read, which no step writes; the weights are the last step's
+  await_previous();
+  let_next_start();
+  {
+    const uint4 *src = reinterpret_cast<const uint4 *>(wimg);
+    uint4 *dst = reinterpret_cast<uint4 *>(smem);
+    for (int q = tid; q < MLP_IMG_BYTES / 16; q += TT_THREADS) dst[q] = src[q];
+    for (int q = tid; q < 387; q += TT_THREADS)
+      bias[q] = params[q < 128 ? MLP_OFF_B1 + q : q < 256 ? MLP_OFF_B2 + q - 128 : q < 384 ? MLP_OFF_B3 + q - 256
+                                                                                       : MLP_OFF_B4 + q - 384];
+  }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -241,30 +271,36 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
   };
   // hidden-layer epilogue: H = bf16(SiLU(C + b)) into the activation buffer
   auto epi_hidden = [&](unsigned cc, const float *bl) {
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      const int col = 32 * cg + 16 * c;
-      float v[16];
-      tmem_ld16(tl + cc + (unsigned)col, v);
-      unsigned w[8];
+    unsigned v[32];
+    tmem_ld32_issue(tl + cc + 32u * cg, v);
+    tmem_wait_ld32(v);
+    const float *bc = bl + 32 * cg;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) w[q] = bf16x2(silu(v[2 * q] + bl[col + 2 * q]), silu(v[2 * q + 1] + bl[col + 2 * q + 1]));
-      *reinterpret_cast<uint4 *>(smem + TT_SM_H + op_off(row, col, 2048)) = make_uint4(w[0], w[1], w[2], w[3]);
-      *reinterpret_cast<uint4 *>(smem + TT_SM_H + op_off(row, col + 8, 2048)) = make_uint4(w[4], w[5], w[6], w[7]);
+    for (int h = 0; h < 4; ++h) {
+      unsigned w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = 8 * h + 2 * q;
+        w[q] = bf16x2(silu(__uint_as_float(v[o]) + bc[o]), silu(__uint_as_float(v[o + 1]) + bc[o + 1]));
+      }
+      *reinterpret_cast<uint4 *>(smem + TT_SM_H + op_off(row, 32 * cg + 8 * h, 2048)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   };
   // backward epilogue: G = dH * SiLU'(C + b) (FP32) into the gradient buffer as bfloat16, and
   // the warp's column sums of G into red[quarter][column]
   auto epi_back = [&](unsigned dc, unsigned cc, const float *bl) {
-#pragma unroll 1
+    unsigned dv[32], zv[32];
+    tmem_ld32_issue(tl + dc + 32u * cg, dv);
+    tmem_ld32_issue(tl + cc + 32u * cg, zv);
+    tmem_wait_ld32(dv);
+    tmem_wait_ld32(zv);
+#pragma unroll
     for (int c = 0; c < 2; ++c) {
       const int col = 32 * cg + 16 * c;
-      float dv[16], zv[16];
-      tmem_ld16(tl + dc + (unsigned)col, dv);
-      tmem_ld16(tl + cc + (unsigned)col, zv);
       float g[16];
 #pragma unroll
-      for (int q = 0; q < 16; ++q) g[q] = dv[q] * silu_grad(zv[q] + bl[col + q]);
+      for (int q = 0; q < 16; ++q)
+        g[q] = __uint_as_float(dv[16 * c + q]) * silu_grad(__uint_as_float(zv[16 * c + q]) + bl[col + q]);
       unsigned w[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) w[q] = bf16x2(g[2 * q], g[2 * q + 1]);
@@ -276,15 +312,12 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
   };
   // this thread's 32 columns of a 128 x 128 dW in the working columns, as row `row` of W
   auto store_dw = [&](int off) {
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      const int col = 32 * cg + 16 * c;
-      float v[16];
-      tmem_ld16(tl + TT_D + (unsigned)col, v);
-      float4 *dst = reinterpret_cast<float4 *>(prt + off + row * 128 + col);
+    unsigned v[32];
+    tmem_ld32_issue(tl + TT_D + 32u * cg, v);
+    tmem_wait_ld32(v);
+    uint4 *dst = reinterpret_cast<uint4 *>(prt + off + row * 128 + 32 * cg);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-    }
+    for (int q = 0; q < 8; ++q) dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
   };
   // bias gradient of a hidden layer: the four warps' column sums in fixed order
   auto store_db = [&](int off) {
@@ -450,6 +483,8 @@ __global__ void k_train_update(const float *__restrict__ part, int tiles, const 
                                float *__restrict__ v, unsigned char *__restrict__ wimg, float *__restrict__ loss_out,
                                int adam, float lr, float c1, float c2) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  await_previous();
+  let_next_start();
   if (q == 0 && loss_out) {
     float l = 0.f;
     for (int t = 0; t < tiles; ++t) l += loss_part[t];
@@ -514,15 +549,15 @@ void mlp_train_step(const unsigned char *wimg, const float *params, const float 
     cudaFuncSetAttribute(k_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SM_LAUNCH);
     attr_device = dev;
   }
-  k_train_tc<<<(unsigned)mlp_train_tiles(B), TT_THREADS, TT_SM_LAUNCH, s>>>(
-      wimg, params, xs, ts, n_samples, seed, step, hashed, B, sc[0], sc[1], sc[2], part, loss_part, err,
-      stall_test ? 1024ull : GT_WAIT_LIMIT, stall_test);
+  launch_after(k_train_tc, (unsigned)mlp_train_tiles(B), TT_THREADS, TT_SM_LAUNCH, s, wimg, params, xs, ts, n_samples,
+               seed, step, hashed, B, sc[0], sc[1], sc[2], part, loss_part, err, stall_test ? 1024ull : GT_WAIT_LIMIT,
+               stall_test);
 }
 void mlp_train_update(const float *part, int tiles, const float *loss_part, float *params, float *grads, float *m,
                       float *v, unsigned char *wimg, float *loss_out, int adam, float lr, float c1, float c2,
                       cudaStream_t s) {
-  k_train_update<<<blocks_for(MLP_NPARAM, 256), 256, 0, s>>>(part, tiles, loss_part, params, grads, m, v, wimg,
-                                                             loss_out, adam, lr, c1, c2);
+  launch_after(k_train_update, blocks_for(MLP_NPARAM, 256), 256, 0, s, part, tiles, loss_part, params, grads, m, v, wimg,
+               loss_out, adam, lr, c1, c2);
 }
 
 namespace {

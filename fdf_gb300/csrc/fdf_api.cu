@@ -696,8 +696,8 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
     CU(cudaEventRecord(ctx->ev_scan, s));
     CU(cudaStreamWaitEvent(ctx->side, ctx->ev_scan, 0));
     c0 = prof ? record_event(ctx, ctx->side) : 0;
-    if (f32)   // FP32 arithmetic is cheap: every node, no occupancy test
-      launch_center_to_corner32(ctx->ucat32, g, ctx->corner32, nullptr, nullptr, ctx->side);
+    if (f32)   // every node, no occupancy test
+      launch_center_to_corner32(ctx->ucat32, g, ctx->corner32, ctx->side);
     else
       launch_center_to_corner(ctx->ucat, g, ctx->corner, ctx->cell_start, &ctx->cnt->nodes_total, ctx->side);
     c1 = prof ? record_event(ctx, ctx->side) : 0;
@@ -723,7 +723,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
     // no deposit
   } else if (f32) {
     float *m = ctx->momentum ? ctx->mom32 : nullptr;
-    launch_deposit32(dst, g, ctx->cell_start, ctx->volume, ctx->count32, ctx->avg32, ctx->fi32, ctx->fj32, ctx->fk32,
+    launch_deposit32(dst, ctx->cap, g, ctx->cell_start, ctx->volume, ctx->count32, ctx->avg32, ctx->fi32, ctx->fj32, ctx->fk32,
                      m, m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, s);
   } else {
     double *m = ctx->momentum ? ctx->mom : nullptr;
@@ -842,7 +842,7 @@ int fdf_InterpolateAllFieldsToSwarm(FdfContext *ctx) {
   const GridDims &g = ctx->g;
   SwarmBuf &b = ctx->buf[ctx->cur];
   if (form_is32(ctx->swarm_form)) {
-    launch_center_to_corner32(ctx->ucat32, g, ctx->corner32, nullptr, nullptr, ctx->stream);
+    launch_center_to_corner32(ctx->ucat32, g, ctx->corner32, ctx->stream);
     launch_gather_interp32(b, b, ctx->cap, g, ctx->corner32, nullptr, ctx->cell_start, ctx->cnt, ctx->stream,
                            INTERP_KEEP);
   } else {
@@ -865,7 +865,7 @@ int fdf_ScatterAllParticleFieldsToEulerFields(FdfContext *ctx) {
   const long long nfi = (g.IM + 1LL) * g.JM * g.KM, nfj = g.IM * (g.JM + 1LL) * g.KM;
   if (form_is32(ctx->swarm_form)) {
     float *m = ctx->momentum ? ctx->mom32 : nullptr;
-    launch_deposit32(b, g, ctx->cell_start, ctx->volume, ctx->count32, ctx->avg32, ctx->fi32, ctx->fj32, ctx->fk32,
+    launch_deposit32(b, ctx->cap, g, ctx->cell_start, ctx->volume, ctx->count32, ctx->avg32, ctx->fi32, ctx->fj32, ctx->fk32,
                      m, m ? m + 3 * nfi : nullptr, m ? m + 3 * (nfi + nfj) : nullptr, ctx->stream);
   } else {
     double *m = ctx->momentum ? ctx->mom : nullptr;

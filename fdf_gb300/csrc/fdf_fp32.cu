@@ -358,44 +358,57 @@ __global__ void __launch_bounds__(256) k_resort_keys(SwarmBuf b, GridDims g, int
   block_flush_counts(m, cnt);
 }
 
-// Corner field in FP32: mean of the valid adjacent cells (nodes next to occupied cells).
-__global__ void k_center_to_corner32(const float *__restrict__ ucat, GridDims g, float *__restrict__ corner,
-                                     const unsigned int *__restrict__ cell_start, unsigned long long *nodes_done) {
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const bool work = q < g.Nn;
-  int i = 0, j = 0, k = 0;
-  if (work) node_ijk(g, (unsigned int)q, i, j, k);
-  if (cell_start) {
-    bool need = false;
-    if (work)
-      for (int dk = -1; dk <= 0 && !need; ++dk)
-        for (int dj = -1; dj <= 0 && !need; ++dj)
-          for (int di = -1; di <= 0 && !need; ++di) {
-            int ck = k + dk, cj = j + dj, ci = i + di;
-            if (ci < 0 || ci >= g.IM || cj < 0 || cj >= g.JM || ck < 0 || ck >= g.KM) continue;
-            long long c = ((long long)ck * g.JM + cj) * g.IM + ci;
-            need = __ldg(cell_start + c + 1) > __ldg(cell_start + c);
-          }
-    if (nodes_done) block_add_u64(need ? 1ull : 0ull, nodes_done);
-    if (!need) return;
+// Corner field in FP32: mean of the valid adjacent cells.  A thread carries NK nodes up the k
+// direction and keeps each layer's four cells for the next node: 12 loads a node instead of 24, and the
+// neighbours' indices and bounds once a column.  (One node per thread was bound by issue: 296
+// instructions a node, 73 % of the issue slots.  14M cells beside the sort: 182 us then, 108 now; columns
+// of 8 nodes 104, of 2 125, but a small grid then has too few threads.)
+template <int NK>
+__global__ void __launch_bounds__(256) k_center_to_corner32(const float *__restrict__ ucat, GridDims g,
+                                                           float *__restrict__ corner) {
+  const unsigned int layer = (unsigned int)(g.IM + 1) * (unsigned int)(g.JM + 1);
+  const unsigned int across_blocks = (layer + 255u) / 256u, up = blockIdx.x / across_blocks;
+  const unsigned int q = (blockIdx.x - up * across_blocks) * 256u + threadIdx.x;
+  if (q >= layer) return;
+  const unsigned int j = g.fMX.div(q), i = q - j * (unsigned int)(g.IM + 1);
+  const unsigned int IM = g.IM, JM = g.JM, KM = g.KM, k0 = up * NK;
+  // the column's four cells of a layer, in (dj, di) order
+  const bool in[4] = {j > 0 && i > 0, j > 0 && i < IM, j < JM && i > 0, j < JM && i < IM};
+  const unsigned int at[4] = {(j - 1) * IM + i - 1, (j - 1) * IM + i, j * IM + i - 1, j * IM + i};
+  const int across = (in[0] ? 1 : 0) + (in[1] ? 1 : 0) + (in[2] ? 1 : 0) + (in[3] ? 1 : 0);
+  float lo[3][4], hi[3][4];   // the layers below and above the node
+  auto load = [&](unsigned int kc, float (&v)[3][4]) {
+    const unsigned int base = kc * (IM * JM);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[d][e] = kc < KM && in[e] ? __ldg(ucat + d * g.Nc + (base + at[e])) : 0.f;
+  };
+  load(k0 - 1u, lo);   // k0 = 0: no such layer
+#pragma unroll
+  for (int m = 0; m < NK; ++m) {
+    const unsigned int k = k0 + m;
+    if (k > KM) return;
+    load(k, hi);
+    const int cells = ((k > 0 ? 1 : 0) + (k < KM ? 1 : 0)) * across;
+    const float r = cells == 8 ? 0.125f : cells == 4 ? 0.25f : cells == 2 ? 0.5f : cells == 1 ? 1.0f : 0.0f;
+    const unsigned int node = k * layer + q;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      // the sum of the valid cells in order, from zero; a cell that is not there adds zero to it (a sum
+      // that is -0 by then is +0 after the first addition either way)
+      float t = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) t += lo[d][e];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) t += hi[d][e];
+      corner[d * g.Nn + node] = t * r;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) lo[d][e] = hi[d][e];
   }
-  if (!work) return;
-  float sx = 0.f, sy = 0.f, sz = 0.f;
-  int count = 0;
-#pragma unroll
-  for (int dk = -1; dk <= 0; ++dk)
-#pragma unroll
-    for (int dj = -1; dj <= 0; ++dj)
-#pragma unroll
-      for (int di = -1; di <= 0; ++di) {
-        const int ck = k + dk, cj = j + dj, ci = i + di;
-        if (ci < 0 || ci >= g.IM || cj < 0 || cj >= g.JM || ck < 0 || ck >= g.KM) continue;
-        const long long c = ((long long)ck * g.JM + cj) * g.IM + ci;
-        sx += __ldg(ucat + c); sy += __ldg(ucat + g.Nc + c); sz += __ldg(ucat + 2 * g.Nc + c);
-        ++count;
-      }
-  const float r = count == 8 ? 0.125f : count == 4 ? 0.25f : count == 2 ? 0.5f : count == 1 ? 1.0f : 0.0f;
-  corner[q] = sx * r; corner[g.Nn + q] = sy * r; corner[2 * g.Nn + q] = sz * r;
 }
 
 __global__ void __launch_bounds__(256) k_gather_interp32(SwarmBuf src, SwarmBuf dst, GridDims g,
@@ -469,8 +482,8 @@ struct KSum {
 
 // Resident 256-thread blocks per SM the volume and the momentum deposits are compiled for.  The
 // per-node chains wait on their loads, so 2048 resident threads (32 registers, a few spilled)
-// beat the 48-register default for the volume deposit: 0.617 -> 0.532 ms per 64M-particle step
-// (0.558 at 5 blocks, 0.550 at 6); 1024 (64 registers) beat 768 (80) for the momentum deposit:
+// beat the 48-register default for the volume deposit (64-bit indices: 0.617 -> 0.532 ms per
+// 64M-particle step; 0.558 at 5 blocks, 0.550 at 6); 1024 (64 registers) beat 768 (80) for the momentum deposit:
 // 2.95 -> 2.88 ms per 128M-particle step.
 #ifndef FDF_DEP32_MIN_BLOCKS
 #define FDF_DEP32_MIN_BLOCKS 8
@@ -478,97 +491,102 @@ struct KSum {
 #ifndef FDF_DEPM32_MIN_BLOCKS
 #define FDF_DEPM32_MIN_BLOCKS 4
 #endif
-template <bool MOM>
-__global__ void __launch_bounds__(256, MOM ? FDF_DEPM32_MIN_BLOCKS : FDF_DEP32_MIN_BLOCKS) k_deposit32(SwarmBuf b, GridDims g, const unsigned int *__restrict__ cs,
-                                                   float third, float *__restrict__ count, float *__restrict__ avg,
-                                                   float *__restrict__ fi, float *__restrict__ fj,
-                                                   float *__restrict__ fk, float *__restrict__ mi,
-                                                   float *__restrict__ mj, float *__restrict__ mk) {
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q >= g.Nn) return;
-  const int IM = g.IM, JM = g.JM, KM = g.KM;
-  int i, j, k;
-  node_ijk(g, (unsigned int)q, i, j, k);
-  const bool is_cell = i < IM && j < JM && k < KM;
-  const long long c = ((long long)k * JM + j) * IM + i;
-  int s0 = 0, s1 = 0;
-  if (is_cell) { s0 = (int)__ldg(cs + c); s1 = (int)__ldg(cs + c + 1); }
+// CH: particles of a segment whose loads are issued before their in-order adds (the own cell's half of
+// that).  Where the particles are fewer than the cells most segments hold none or one, and the chunk's
+// idle entries only take issue slots, which bound this kernel: 6M particles in 14M cells 218 us with 4,
+// 232 with 8; above, the loads' latency counts, 64M particles 477 us with 8, 495 with 4.  (Every index
+// is 32 bits: with 64-bit ones a node took 550 instructions, 268 and 521 us.)
+template <bool MOM, int CH>
+__global__ void __launch_bounds__(256, MOM ? FDF_DEPM32_MIN_BLOCKS : FDF_DEP32_MIN_BLOCKS)
+    k_deposit32(SwarmBuf b, GridDims g, const unsigned int *__restrict__ cs, float third, float *__restrict__ count,
+                float *__restrict__ avg, float *__restrict__ fi, float *__restrict__ fj, float *__restrict__ fk,
+                float *__restrict__ mi, float *__restrict__ mj, float *__restrict__ mk) {
+  const unsigned int q = blockIdx.x * blockDim.x + threadIdx.x;   // below 2^31, as every index here
+  if (q >= (unsigned int)g.Nn) return;
+  const unsigned int IM = g.IM, JM = g.JM, KM = g.KM;
+  unsigned int i, j, k;
+  {
+    int ii, jj, kk;
+    node_ijk(g, q, ii, jj, kk);
+    i = ii; j = jj; k = kk;
+  }
+  const unsigned int row = k * JM + j, c = row * IM + i;   // the cell's row and id, were (i, j, k) a cell
+  const bool face_i = j < JM && k < KM, face_j = i < IM && k < KM, face_k = i < IM && j < JM;
+  const bool is_cell = face_i && i < IM;
+  unsigned int s0 = 0u, s1 = 0u;
+  if (face_i) s0 = s1 = __ldg(cs + c);   // (i = IM: where the row's last cell ends)
+  if (is_cell) s1 = __ldg(cs + c + 1u);
   // per face the lower cell's segment first, then this cell's; the three lower segments run
   // first and this cell's segment then feeds the P sum and the three upper parts in one pass
   // (every accumulator receives its values in the same order as face by face)
-  const long long nfi = (IM + 1LL) * JM * KM, nfj = IM * (JM + 1LL) * KM, nfk = (long long)IM * JM * (KM + 1LL);
-  const bool face_i = j < JM && k < KM, face_j = i < IM && k < KM, face_k = i < IM && j < JM;
   KSum acc[3], mm[3][3];
-  // Each segment is read in chunks of DCH particles, all loads of a chunk issued before its
-  // in-order adds, so one load latency serves the chunk instead of each particle.
-  constexpr int DCH = MOM ? 4 : 8;
-  auto lower = [&](int f, const float *__restrict__ wgt, long long lc) {
-    const int l0 = (int)__ldg(cs + lc), l1 = (int)__ldg(cs + lc + 1);
-    for (int s = l0; s < l1; s += DCH) {
-      float a[DCH], u[DCH], v[DCH], w[DCH];
+  auto lower = [&](int f, const float *__restrict__ wgt, unsigned int l0, unsigned int l1) {
+    for (unsigned int s = l0; s < l1; s += CH) {
+      float a[CH], u[CH], v[CH], w[CH];
 #pragma unroll
-      for (int q = 0; q < DCH; ++q) {
-        const bool in = s + q < l1;
-        a[q] = in ? __ldg(wgt + s + q) : 0.f;
+      for (int e = 0; e < CH; ++e) {
+        const bool in = s + e < l1;
+        a[e] = in ? __ldg(wgt + s + e) : 0.f;
         if (MOM) {
-          u[q] = in ? __ldg(b.uf + s + q) : 0.f;
-          v[q] = in ? __ldg(b.vf + s + q) : 0.f;
-          w[q] = in ? __ldg(b.wf + s + q) : 0.f;
+          u[e] = in ? __ldg(b.uf + s + e) : 0.f;
+          v[e] = in ? __ldg(b.vf + s + e) : 0.f;
+          w[e] = in ? __ldg(b.wf + s + e) : 0.f;
         }
       }
 #pragma unroll
-      for (int q = 0; q < DCH; ++q) {
-        if (s + q >= l1) break;
-        const float fr = a[q] * third;
+      for (int e = 0; e < CH; ++e) {
+        if (s + e >= l1) break;
+        const float fr = a[e] * third;
         acc[f].add(fr);
-        if (MOM) { mm[f][0].add(fr * u[q]); mm[f][1].add(fr * v[q]); mm[f][2].add(fr * w[q]); }
+        if (MOM) { mm[f][0].add(fr * u[e]); mm[f][1].add(fr * v[e]); mm[f][2].add(fr * w[e]); }
       }
     }
   };
-  if (face_i && i > 0) lower(0, b.a1f, c - 1);
-  if (face_j && j > 0) lower(1, b.a2f, ((long long)k * JM + (j - 1)) * IM + i);
-  if (face_k && k > 0) lower(2, b.a3f, ((long long)(k - 1) * JM + j) * IM + i);
+  if (face_i && i > 0) lower(0, b.a1f, __ldg(cs + c - 1u), s0);
+  if (face_j && j > 0) lower(1, b.a2f, __ldg(cs + c - IM), __ldg(cs + c - IM + 1u));
+  if (face_k && k > 0) lower(2, b.a3f, __ldg(cs + c - IM * JM), __ldg(cs + c - IM * JM + 1u));
   KSum sum;
-  constexpr int OCH = 4;
-  for (int s = s0; s < s1; s += OCH) {
+  constexpr int OCH = MOM ? CH : (CH + 1) / 2;
+  for (unsigned int s = s0; s < s1; s += OCH) {
     float P[OCH], w[OCH][3], u[OCH], v[OCH], ww[OCH];
 #pragma unroll
-    for (int q = 0; q < OCH; ++q) {
-      const bool in = s + q < s1;
-      P[q] = in ? __ldg(b.Pf + s + q) : 0.f;
-      w[q][0] = in ? __ldg(b.a1f + s + q) : 0.f;
-      w[q][1] = in ? __ldg(b.a2f + s + q) : 0.f;
-      w[q][2] = in ? __ldg(b.a3f + s + q) : 0.f;
+    for (int e = 0; e < OCH; ++e) {
+      const bool in = s + e < s1;
+      P[e] = in ? __ldg(b.Pf + s + e) : 0.f;
+      w[e][0] = in ? __ldg(b.a1f + s + e) : 0.f;
+      w[e][1] = in ? __ldg(b.a2f + s + e) : 0.f;
+      w[e][2] = in ? __ldg(b.a3f + s + e) : 0.f;
       if (MOM) {
-        u[q] = in ? __ldg(b.uf + s + q) : 0.f;
-        v[q] = in ? __ldg(b.vf + s + q) : 0.f;
-        ww[q] = in ? __ldg(b.wf + s + q) : 0.f;
+        u[e] = in ? __ldg(b.uf + s + e) : 0.f;
+        v[e] = in ? __ldg(b.vf + s + e) : 0.f;
+        ww[e] = in ? __ldg(b.wf + s + e) : 0.f;
       }
     }
 #pragma unroll
-    for (int q = 0; q < OCH; ++q) {
-      if (s + q >= s1) break;
-      sum.add(P[q]);
+    for (int e = 0; e < OCH; ++e) {
+      if (s + e >= s1) break;
+      sum.add(P[e]);
 #pragma unroll
       for (int f = 0; f < 3; ++f) {
-        const float fr = (1.f - w[q][f]) * third;
+        const float fr = (1.f - w[e][f]) * third;
         acc[f].add(fr);
-        if (MOM) { mm[f][0].add(fr * u[q]); mm[f][1].add(fr * v[q]); mm[f][2].add(fr * ww[q]); }
+        if (MOM) { mm[f][0].add(fr * u[e]); mm[f][1].add(fr * v[e]); mm[f][2].add(fr * ww[e]); }
       }
     }
   }
   {
-    const int nc = s1 - s0;
+    const unsigned int nc = s1 - s0;
     count[q] = (float)nc;
     avg[q] = nc > 0 ? sum.value() / (float)nc : 0.f;
   }
-  auto store = [&](int f, float *vol, float *mom, long long nf, long long fidx) {
-    vol[fidx] = acc[f].value();
-    if (MOM) { mom[fidx] = mm[f][0].value(); mom[nf + fidx] = mm[f][1].value(); mom[2 * nf + fidx] = mm[f][2].value(); }
+  auto store = [&](int f, float *vol, float *mom, long long nf, unsigned int at) {
+    vol[at] = acc[f].value();
+    if (MOM) { mom[at] = mm[f][0].value(); mom[nf + at] = mm[f][1].value(); mom[2 * nf + at] = mm[f][2].value(); }
   };
-  if (face_i) store(0, fi, mi, nfi, ((long long)k * JM + j) * (IM + 1) + i);
-  if (face_j) store(1, fj, mj, nfj, ((long long)k * (JM + 1) + j) * IM + i);
-  if (face_k) store(2, fk, mk, nfk, c);
+  // (row (IM + 1) + i, (k (JM + 1) + j) IM + i, c)
+  if (face_i) store(0, fi, mi, MOM ? (IM + 1LL) * JM * KM : 0, c + row);
+  if (face_j) store(1, fj, mj, MOM ? IM * (JM + 1LL) * KM : 0, c + k * IM);
+  if (face_k) store(2, fk, mk, MOM ? (long long)IM * JM * (KM + 1LL) : 0, c);
 }
 
 __global__ void k_from_aos32(const double *__restrict__ pos, const double *__restrict__ vel,
@@ -769,9 +787,11 @@ void launch_locate32_path(const SwarmBuf &b, int n_cap, GridDims g, const float 
       FDF_PATH_LOOKAHEAD);
 }
 
-void launch_center_to_corner32(const float *ucat, GridDims g, float *corner, const unsigned int *cell_start,
-                               unsigned long long *nodes_done, cudaStream_t s) {
-  k_center_to_corner32<<<blocks_for(g.Nn, 256), 256, 0, s>>>(ucat, g, corner, cell_start, nodes_done);
+void launch_center_to_corner32(const float *ucat, GridDims g, float *corner, cudaStream_t s) {
+  constexpr int NK = 4;
+  const unsigned int layer = (unsigned int)(g.IM + 1) * (unsigned int)(g.JM + 1);
+  const unsigned int blocks = blocks_for(layer, 256) * (unsigned int)((g.KM + NK) / NK);   // KM + 1 layers of nodes
+  k_center_to_corner32<NK><<<blocks, 256, 0, s>>>(ucat, g, corner);
 }
 
 void launch_advect32(const SwarmBuf &b, int n_cap, double dt, DevCounters *cnt, cudaStream_t s) {
@@ -795,14 +815,17 @@ void launch_gather_interp32(const SwarmBuf &src, const SwarmBuf &dst, int n_cap,
   k_gather_interp32<<<blocks_for(n_cap, 256), 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode);
 }
 
-void launch_deposit32(const SwarmBuf &b, GridDims g, const unsigned int *cell_start, double volume, float *count,
+void launch_deposit32(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, float *count,
                       float *avg, float *fi, float *fj, float *fk, float *mi, float *mj, float *mk, cudaStream_t s) {
+  constexpr int th = 256;
+  const unsigned int blocks = blocks_for(g.Nn, th);
+  const float third = (float)(volume / 3.0);
   if (mi)
-    k_deposit32<true><<<blocks_for(g.Nn, 256), 256, 0, s>>>(b, g, cell_start, (float)(volume / 3.0), count, avg, fi,
-                                                            fj, fk, mi, mj, mk);
+    k_deposit32<true, 4><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
+  else if (n_cap <= g.Nc)
+    k_deposit32<false, 4><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, nullptr, nullptr, nullptr);
   else
-    k_deposit32<false><<<blocks_for(g.Nn, 256), 256, 0, s>>>(b, g, cell_start, (float)(volume / 3.0), count, avg, fi,
-                                                             fj, fk, nullptr, nullptr, nullptr);
+    k_deposit32<false, 8><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, nullptr, nullptr, nullptr);
 }
 
 void launch_swarm_from_aos32(const double *pos, const double *vel, const double *wgt, const double *P,

@@ -269,12 +269,11 @@ void launch_locate32_path(const SwarmBuf &b, int n_cap, GridDims g, const float 
                           const double *bbox, const float *fbox, int drop_removed, DevCounters *cnt,
                           unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
                           const unsigned int *pending, const int *guess, int num_sms, cudaStream_t s);
-void launch_center_to_corner32(const float *ucat, GridDims g, float *corner, const unsigned int *cell_start,
-                               unsigned long long *nodes_done, cudaStream_t s);
+void launch_center_to_corner32(const float *ucat, GridDims g, float *corner, cudaStream_t s);
 void launch_gather_interp32(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const float *corner,
                             const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt,
                             cudaStream_t s, int mode = GATHER_INTERP);
-void launch_deposit32(const SwarmBuf &b, GridDims g, const unsigned int *cell_start, double volume, float *count,
+void launch_deposit32(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, float *count,
                       float *avg, float *fi, float *fj, float *fk, float *mi, float *mj, float *mk, cudaStream_t s);
 void launch_swarm_from_aos32(const double *pos, const double *vel, const double *wgt, const double *P,
                              const long long *cell3, const long long *pid, const long long *status, int n, GridDims g,

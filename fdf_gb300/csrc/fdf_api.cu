@@ -312,6 +312,7 @@ static void swarm_replaced(FdfContext *ctx) {
   ctx->swarm_form = ctx->form;
   ctx->swarm_set = true;
   ctx->layout_ok = false;
+  ctx->unsorted = 0;
 }
 
 // The swarm buffers from particle `off` on.
@@ -489,6 +490,7 @@ int fdf_SeedParticles(FdfContext *ctx, int64_t n, uint64_t seed, int start_in_ge
   CU(cudaMemcpyAsync(ctx->cnt, &c, sizeof(c), cudaMemcpyHostToDevice, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   swarm_replaced(ctx);
+  ctx->unsorted = n;
   return FDF_SUCCESS;
 }
 
@@ -644,6 +646,13 @@ int read_info(FdfContext *ctx, FdfStepInfo *info) {
   return FDF_SUCCESS;
 }
 
+// From this many particles on, a seeded swarm's first sort gathers one record per particle, packed in a
+// pass of its own, instead of an element of each array: in no order of cells every element costs a
+// sector and a page of its own.  At 64M particles 13.6 -> 4.0 ms (FP32 form), at 16M 3.07 -> 0.95 (plain
+// 3.68 -> 1.89), at 4M 537 -> 227 us, at 2M 186 -> 133; where the arrays fit in L2 the pass is only
+// extra: 82 -> 88 us at 1M, 55 -> 61 at 500k.
+constexpr int64_t PACK_MIN = 3 << 19;
+
 // The shared pipeline of the initial setup (advect=0, drop=0) and a step (1, 1); locate_only:
 // the walk and the re-sort alone (fdf_LocateAllParticlesInGrid), no interpolation or deposit.
 int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool locate_only = false) {
@@ -713,7 +722,17 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
   if (!locate_only) CU(cudaStreamWaitEvent(s, ctx->ev_corner, 0));
   size_t e3 = prof ? record_event(ctx, s) : 0;
   const int gmode = locate_only ? GATHER_COPY : GATHER_INTERP;
-  if (f32)
+  const bool packed = !drop && !locate_only && ctx->unsorted >= PACK_MIN;
+  if (packed) {
+    static_assert(FDF_REC_BYTES <= 120, "the records share the transfers' staging buffer");
+    if (f32)
+      launch_gather_interp32_packed(src, dst, ctx->cap, g, ctx->corner32, ctx->perm, ctx->cell_start, ctx->cnt,
+                                    ctx->staging, s);
+    else
+      launch_gather_interp_packed(src, dst, ctx->cap, g, ctx->corner, ctx->perm, ctx->cell_start, ctx->cnt,
+                                  ctx->staging, s);
+    ctx->launches += 1;
+  } else if (f32)
     launch_gather_interp32(src, dst, ctx->cap, g, ctx->corner32, ctx->perm, ctx->cell_start, ctx->cnt, s, gmode);
   else
     launch_gather_interp(src, dst, ctx->cap, g, ctx->corner, ctx->perm, ctx->cell_start, ctx->cnt, s, gmode);
@@ -752,6 +771,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
   CHECK_LAUNCH();
   ctx->cur = 1 - ctx->cur;
   ctx->layout_ok = true;
+  ctx->unsorted = 0;
   ctx->launches += locate_only ? 2 : 4;   // slots, gather; corner field, deposit
   return info ? read_info(ctx, info) : FDF_SUCCESS;
 }
@@ -781,6 +801,7 @@ int resort(FdfContext *ctx, int remove_lost, int remove_oob, int64_t *removed_lo
   CHECK_LAUNCH();
   ctx->cur = 1 - ctx->cur;
   ctx->layout_ok = true;
+  ctx->unsorted = 0;
   DevCounters c{};
   CU(cudaMemcpyAsync(&c, ctx->cnt, DEVCOUNTERS_HEAD, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
@@ -1143,6 +1164,7 @@ static int step_on_stream(FdfContext *ctx, int settled) {
   CU(cudaGraphLaunch(ctx->step_graph[parity], ctx->stream));
   ctx->cur = 1 - parity;
   ctx->layout_ok = true;
+  ctx->unsorted = 0;
   ctx->out_form = ctx->swarm_form;
   ctx->out_momentum = ctx->momentum;
   ctx->launches += ctx->graph_launches;

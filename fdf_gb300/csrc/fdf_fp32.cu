@@ -411,11 +411,27 @@ __global__ void __launch_bounds__(256) k_center_to_corner32(const float *__restr
   }
 }
 
+// What the gather takes of a particle, as one aligned 64-byte record: positions, pid | weights, P | cell.
+__global__ void __launch_bounds__(256) k_pack32(SwarmBuf b, const DevCounters *cnt, uint4 *__restrict__ rec) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= cnt->n_sorted) return;
+  const ulonglong2 xy = make_ulonglong2(fdfx::ubits(b.x[p]), fdfx::ubits(b.y[p]));
+  const ulonglong2 zp = make_ulonglong2(fdfx::ubits(b.z[p]), (unsigned long long)b.pid[p]);
+  uint4 *r = rec + 4 * (size_t)p;
+  *reinterpret_cast<ulonglong2 *>(r) = xy;
+  *reinterpret_cast<ulonglong2 *>(r + 1) = zp;
+  r[2] = make_uint4(__float_as_uint(b.a1f[p]), __float_as_uint(b.a2f[p]), __float_as_uint(b.a3f[p]),
+                    __float_as_uint(b.Pf[p]));
+  r[3] = make_uint4((unsigned int)b.cell[p], 0u, 0u, 0u);
+}
+
+// REC: the particles come from k_pack32's records (mode GATHER_INTERP).
+template <bool REC>
 __global__ void __launch_bounds__(256) k_gather_interp32(SwarmBuf src, SwarmBuf dst, GridDims g,
                                                          const float *__restrict__ corner,
                                                          const unsigned int *__restrict__ perm,
                                                          const unsigned int *__restrict__ cell_start,
-                                                         DevCounters *cnt, int mode) {
+                                                         DevCounters *cnt, int mode, const uint4 *__restrict__ rec) {
   const int n = (int)cell_start[g.Nc + 1];
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0) {
@@ -424,14 +440,28 @@ __global__ void __launch_bounds__(256) k_gather_interp32(SwarmBuf src, SwarmBuf 
   }
   if (s >= n) return;
   const unsigned int p = perm ? perm[s] : (unsigned int)s;
-  const int cell = src.cell[p];
-  float a1 = src.a1f[p], a2 = src.a2f[p], a3 = src.a3f[p];
-  const unsigned char st = src.status[p];
-  dst.x[s] = src.x[p]; dst.y[s] = src.y[p]; dst.z[s] = src.z[p];
+  int cell;
+  float a1, a2, a3;
+  unsigned char st = 0;
+  if (REC) {
+    const uint4 *r = rec + 4 * (size_t)p;
+    const ulonglong2 xy = *reinterpret_cast<const ulonglong2 *>(r), zp = *reinterpret_cast<const ulonglong2 *>(r + 1);
+    const uint4 wp = r[2];
+    cell = (int)r[3].x;
+    a1 = __uint_as_float(wp.x); a2 = __uint_as_float(wp.y); a3 = __uint_as_float(wp.z);
+    dst.x[s] = __longlong_as_double((long long)xy.x); dst.y[s] = __longlong_as_double((long long)xy.y); dst.z[s] = __longlong_as_double((long long)zp.x);
+    dst.Pf[s] = __uint_as_float(wp.w);
+    dst.pid[s] = (long long)zp.y;
+  } else {
+    cell = src.cell[p];
+    a1 = src.a1f[p]; a2 = src.a2f[p]; a3 = src.a3f[p];
+    st = src.status[p];
+    dst.x[s] = src.x[p]; dst.y[s] = src.y[p]; dst.z[s] = src.z[p];
+    dst.Pf[s] = src.Pf[p];
+    dst.pid[s] = src.pid[p];
+  }
   dst.a1f[s] = a1; dst.a2f[s] = a2; dst.a3f[s] = a3;
-  dst.Pf[s] = src.Pf[p];
-  dst.pid[s] = src.pid[p];
-  if (mode == GATHER_COPY) {
+  if (!REC && mode == GATHER_COPY) {
     dst.uf[s] = src.uf[p]; dst.vf[s] = src.vf[p]; dst.wf[s] = src.wf[p];
     dst.cell[s] = cell;
     dst.status[s] = st;
@@ -440,10 +470,10 @@ __global__ void __launch_bounds__(256) k_gather_interp32(SwarmBuf src, SwarmBuf 
   float ux = 0.f, uy = 0.f, uz = 0.f;
   if (cell < 0) {
     dst.cell[s] = -1;
-    dst.status[s] = mode == GATHER_INTERP ? (unsigned char)ST_LOST : st;
+    dst.status[s] = REC || mode == GATHER_INTERP ? (unsigned char)ST_LOST : st;
   } else {
     dst.cell[s] = cell;
-    dst.status[s] = mode == GATHER_INTERP ? (unsigned char)ST_ACTIVE_AND_LOCATED : st;
+    dst.status[s] = REC || mode == GATHER_INTERP ? (unsigned char)ST_ACTIVE_AND_LOCATED : st;
     int i, j, k;
     cell_ijk(g, (unsigned int)cell, i, j, k);
     a1 = fminf(fmaxf(a1, 0.f), 1.f);   // NaN -> 0 as PetscMax(0, PetscMin(1, NaN))
@@ -812,7 +842,17 @@ void launch_resort_keys(const SwarmBuf &b, int n_cap, GridDims g, int f32, int r
 void launch_gather_interp32(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const float *corner,
                             const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt,
                             cudaStream_t s, int mode) {
-  k_gather_interp32<<<blocks_for(n_cap, 256), 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode);
+  k_gather_interp32<false><<<blocks_for(n_cap, 256), 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode,
+                                                                  nullptr);
+}
+
+void launch_gather_interp32_packed(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const float *corner,
+                                   const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt, void *rec,
+                                   cudaStream_t s) {
+  uint4 *r = static_cast<uint4 *>(rec);
+  k_pack32<<<blocks_for(n_cap, 256), 256, 0, s>>>(src, cnt, r);
+  k_gather_interp32<true><<<blocks_for(n_cap, 256), 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt,
+                                                                 GATHER_INTERP, r);
 }
 
 void launch_deposit32(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, float *count,

@@ -207,6 +207,15 @@ enum { GATHER_COPY = 0, GATHER_INTERP = 1, INTERP_KEEP = 2 };
 void launch_gather_interp(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g,
                           const double *corner, const unsigned int *perm, const unsigned int *cell_start,
                           DevCounters *cnt, cudaStream_t s, int mode = GATHER_INTERP);
+// The same (GATHER_INTERP) by way of one record per particle in rec (FDF_REC_BYTES a particle), for a
+// src in no order of cells.
+#define FDF_REC_BYTES 80
+void launch_gather_interp_packed(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const double *corner,
+                                 const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt, void *rec,
+                                 cudaStream_t s);
+void launch_gather_interp32_packed(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const float *corner,
+                                   const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt, void *rec,
+                                   cudaStream_t s);
 // mi, mj, mk (SoA [3][faces], or nullptr): the momentum deposit, V * velocity split like the volume.
 void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, double *count,
                     double *avg, double *fi, double *fj, double *fk, double *mi, double *mj, double *mk,

@@ -52,6 +52,18 @@ __device__ __forceinline__ void trilinear(double a1, double a2, double a3, Value
   }
 }
 
+// What the gather takes of a particle, as one 16-byte aligned 80-byte record: position, weights, P, pid, cell.
+__global__ void __launch_bounds__(256) k_pack(SwarmBuf b, const DevCounters *cnt, ulonglong2 *__restrict__ rec) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= cnt->n_sorted) return;
+  ulonglong2 *r = rec + 5 * (size_t)p;
+  r[0] = make_ulonglong2(fdfx::ubits(b.x[p]), fdfx::ubits(b.y[p]));
+  r[1] = make_ulonglong2(fdfx::ubits(b.z[p]), fdfx::ubits(b.a1[p]));
+  r[2] = make_ulonglong2(fdfx::ubits(b.a2[p]), fdfx::ubits(b.a3[p]));
+  r[3] = make_ulonglong2(fdfx::ubits(b.P[p]), (unsigned long long)b.pid[p]);
+  r[4] = make_ulonglong2((unsigned long long)(long long)b.cell[p], 0ull);
+}
+
 // Sorted slot s takes the particle from slot perm[s] of the previous order, then
 // interpolates ucat to it: ComputeTrilinearWeights (interpolation.c:839-864) and
 // TrilinearInterpolation_Vector (:957-1042) from the node-averaged field, with
@@ -59,11 +71,13 @@ __device__ __forceinline__ void trilinear(double a1, double a2, double a3, Value
 // 2048 resident threads: the products' integer chains and the sums' FP64 chains wait on one another,
 // so resident warps beat the spills of 32 registers (64M particles 4.66 ms; 4.94 at 1536 threads, 5.0 at
 // 1280, 5.5 at the compiler's choice of 48 registers).
+// REC: the particles come from k_pack's records (mode GATHER_INTERP).
+template <bool REC>
 __global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf dst, GridDims g,
                                                        const double *__restrict__ corner,
                                                        const unsigned int *__restrict__ perm,
                                                        const unsigned int *__restrict__ cell_start,
-                                                       DevCounters *cnt, int mode) {
+                                                       DevCounters *cnt, int mode, const ulonglong2 *__restrict__ rec) {
   const int n = (int)cell_start[g.Nc + 1];
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0) {   // the new sizes, read by the next step
@@ -72,14 +86,27 @@ __global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf
   }
   if (s >= n) return;
   const unsigned int p = perm ? perm[s] : (unsigned int)s;
-  const int cell = src.cell[p];
-  double a1 = src.a1[p], a2 = src.a2[p], a3 = src.a3[p];
-  const unsigned char st = src.status[p];
-  dst.x[s] = src.x[p]; dst.y[s] = src.y[p]; dst.z[s] = src.z[p];
+  int cell;
+  double a1, a2, a3;
+  unsigned char st = 0;
+  if (REC) {
+    const ulonglong2 *r = rec + 5 * (size_t)p;
+    const ulonglong2 xy = r[0], za = r[1], ab = r[2], Pp = r[3];
+    cell = (int)r[4].x;
+    a1 = __longlong_as_double((long long)za.y); a2 = __longlong_as_double((long long)ab.x); a3 = __longlong_as_double((long long)ab.y);
+    dst.x[s] = __longlong_as_double((long long)xy.x); dst.y[s] = __longlong_as_double((long long)xy.y); dst.z[s] = __longlong_as_double((long long)za.x);
+    dst.P[s] = __longlong_as_double((long long)Pp.x);
+    dst.pid[s] = (long long)Pp.y;
+  } else {
+    cell = src.cell[p];
+    a1 = src.a1[p]; a2 = src.a2[p]; a3 = src.a3[p];
+    st = src.status[p];
+    dst.x[s] = src.x[p]; dst.y[s] = src.y[p]; dst.z[s] = src.z[p];
+    dst.P[s] = src.P[p];
+    dst.pid[s] = src.pid[p];
+  }
   dst.a1[s] = a1; dst.a2[s] = a2; dst.a3[s] = a3;
-  dst.P[s] = src.P[p];
-  dst.pid[s] = src.pid[p];
-  if (mode == GATHER_COPY) {
+  if (!REC && mode == GATHER_COPY) {
     dst.u[s] = src.u[p]; dst.v[s] = src.v[p]; dst.w[s] = src.w[p];
     dst.cell[s] = cell;
     dst.status[s] = st;
@@ -88,10 +115,10 @@ __global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf
   double ux = 0.0, uy = 0.0, uz = 0.0;
   if (cell < 0) {
     dst.cell[s] = -1;
-    dst.status[s] = mode == GATHER_INTERP ? (unsigned char)ST_LOST : st;
+    dst.status[s] = REC || mode == GATHER_INTERP ? (unsigned char)ST_LOST : st;
   } else {
     dst.cell[s] = cell;
-    dst.status[s] = mode == GATHER_INTERP ? (unsigned char)ST_ACTIVE_AND_LOCATED : st;
+    dst.status[s] = REC || mode == GATHER_INTERP ? (unsigned char)ST_ACTIVE_AND_LOCATED : st;
     int i, j, k;
     cell_ijk(g, (unsigned int)cell, i, j, k);
     const long long mx = g.IM + 1, my = g.JM + 1;
@@ -407,7 +434,16 @@ void launch_gather_interp(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, G
   int th = 256;
   int blocks = (n_cap + th - 1) / th;
   if (blocks == 0) blocks = 1;
-  k_gather_interp<<<blocks, th, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode);
+  k_gather_interp<false><<<blocks, th, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode, nullptr);
+}
+
+void launch_gather_interp_packed(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const double *corner,
+                                 const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt, void *rec,
+                                 cudaStream_t s) {
+  const unsigned int blocks = n_cap > 0 ? (unsigned int)((n_cap + 255) / 256) : 1u;
+  ulonglong2 *r = static_cast<ulonglong2 *>(rec);
+  k_pack<<<blocks, 256, 0, s>>>(src, cnt, r);
+  k_gather_interp<true><<<blocks, 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, GATHER_INTERP, r);
 }
 
 void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, double *count,

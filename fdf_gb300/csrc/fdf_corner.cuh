@@ -2,46 +2,44 @@
 // (interpolation.c:598-679).  A node averages its valid adjacent cells in (dk, dj, di) order.  The
 // count is a product of per-direction counts of 1 or 2, i.e. 1, 2, 4 or 8, so sum/count is exactly
 // sum*(1/count): both are the correctly rounded value of the same real.  The running sum starts at
-// 0.0; "0.0 + first" is the first value except that a -0.0 becomes +0.0 (add0).
+// 0.0; "0.0 + first" is the first value except that a -0.0 becomes +0.0 (add0).  It is never -0.0 after
+// that, so a cell that is not there can add +0.0: the lanes of a row's ends take the others' path.
 #pragma once
 #include "fdf_internal.cuh"
 #include "fdf_exact.cuh"
 
 namespace fdfx {
 
+// XI, YI, ZI: bit e puts the addition of the e-th cell to that component on the integer pipe (the same
+// bits).
+template <int XI, int YI, int ZI>
 __device__ __forceinline__ void corner_value(const double *__restrict__ ucat, const GridDims &g, int i, int j, int k,
                                              double &ox, double &oy, double &oz) {
-  const double *ux = ucat, *uy = ucat + g.Nc, *uz = ucat + 2 * g.Nc;
+  const unsigned int IM = g.IM, JM = g.JM;
+  const bool i_lo = i > 0, i_hi = i < g.IM, j_lo = j > 0, j_hi = j < g.JM, k_lo = k > 0, k_hi = k < g.KM;
   double sx = 0.0, sy = 0.0, sz = 0.0;
-  int count = 0;
 #pragma unroll
-  for (int dk = -1; dk <= 0; ++dk) {
-    const long long ck = k + dk;
-    if (ck < 0 || ck >= g.KM) continue;
+  for (int r = 0; r < 4; ++r) {
+    const bool row_in = ((r & 2) ? k_hi : k_lo) && ((r & 1) ? j_hi : j_lo);
+    // the row's two cells; the first one's index wraps for i = 0, where it is not read
+    const unsigned int c1 = ((unsigned int)(k - 1 + (r >> 1)) * JM + (unsigned int)(j - 1 + (r & 1))) * IM + (unsigned int)i;
 #pragma unroll
-    for (int dj = -1; dj <= 0; ++dj) {
-      const long long cj = j + dj;
-      if (cj < 0 || cj >= g.JM) continue;
-#pragma unroll
-      for (int di = -1; di <= 0; ++di) {
-        const long long ci = i + di;
-        if (ci < 0 || ci >= g.IM) continue;
-        const long long c = (ck * g.JM + cj) * g.IM + ci;
-        const double vx = __ldg(ux + c), vy = __ldg(uy + c), vz = __ldg(uz + c);
-        if (count == 0) {
-          sx = add0(vx); sy = add0(vy); sz = add0(vz);
-        } else {
-          sx = add(sx, vx); sy = add(sy, vy); sz = add(sz, vz);
-        }
-        ++count;
+    for (int di = 0; di < 2; ++di) {
+      const int e = 2 * r + di;
+      const bool in = row_in && (di ? i_hi : i_lo);
+      const double *u = ucat + (di ? c1 : c1 - 1u);
+      const double vx = in ? __ldg(u) : 0.0, vy = in ? __ldg(u + g.Nc) : 0.0, vz = in ? __ldg(u + 2 * g.Nc) : 0.0;
+      if (e == 0) {
+        sx = add0(vx); sy = add0(vy); sz = add0(vz);
+      } else {
+        sx = (XI >> e & 1) ? add_int(sx, vx) : add(sx, vx);
+        sy = (YI >> e & 1) ? add_int(sy, vy) : add(sy, vy);
+        sz = (ZI >> e & 1) ? add_int(sz, vz) : add(sz, vz);
       }
     }
   }
-  ox = 0.0; oy = 0.0; oz = 0.0;
-  if (count > 0) {
-    const int sh = count == 1 ? 0 : count == 2 ? 1 : count == 4 ? 2 : 3;   // sum * 0.5^sh, exact
-    ox = scale_down(sx, sh); oy = scale_down(sy, sh); oz = scale_down(sz, sh);
-  }
+  const int sh = (int)(i_lo && i_hi) + (int)(j_lo && j_hi) + (int)(k_lo && k_hi);   // sum * 0.5^sh, exact
+  ox = scale_down(sx, sh); oy = scale_down(sy, sh); oz = scale_down(sz, sh);
 }
 
 }  // namespace fdfx

@@ -255,6 +255,47 @@ __device__ __forceinline__ double mul_int(double a, double b) {
   return __longlong_as_double((long long)r);
 }
 
+// a + b, round to nearest even, on the integer pipe: the same bits as __dadd_rn.  Fast path: both
+// normal, the larger one's exponent away from both ends of the range, and no more than 31 leading bits
+// cancelled; a zero adds nothing; the rest takes the hardware addition out of line.
+//
+// In units of 2^-10 of the larger operand's last place: its significand X has its top bit at 62, the
+// smaller one's is shifted right to odd (the last bit set when bits were lost), which leaves the sum's
+// rounding to 53 bits as it was: X is even, and nine bits or more stay below the rounding position
+// unless the shift is at most one place, where nothing is lost.
+static __device__ __noinline__ double add_hw(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double add_int(double a, double b) {
+  unsigned long long x = ubits(a), y = ubits(b);
+  const bool less = (x & ABS_MASK) < (y & ABS_MASK);
+  const unsigned long long big = less ? y : x, small = less ? x : y;
+  const unsigned int xh = (unsigned int)(big >> 32), xl = (unsigned int)big;
+  const unsigned int yh = (unsigned int)(small >> 32), yl = (unsigned int)small;
+  const unsigned int ex = (xh >> 20) & 0x7ffu, ey = (yh >> 20) & 0x7ffu;
+  if (ey == 0u || ex - 64u > 2045u - 64u) {
+    if ((small & ABS_MASK) == 0ull && ex != 0x7ffu)   // plus zero
+      return __longlong_as_double((long long)((big & ABS_MASK) == 0ull ? x & y : big));
+    return add_hw(a, b);
+  }
+  const unsigned long long X =
+      ((unsigned long long)((__funnelshift_l(xl, xh, 10) & 0x3fffffffu) | 0x40000000u) << 32) | (xl << 10);
+  const unsigned long long Y =
+      ((unsigned long long)((__funnelshift_l(yl, yh, 10) & 0x3fffffffu) | 0x40000000u) << 32) | (yl << 10);
+  const unsigned int d = min(ex - ey, 63u);
+  unsigned long long t = Y >> d;
+  if ((t << d) != Y) t |= 1ull;
+  const long long neg = (long long)((int)(xh ^ yh) >> 31);   // all ones when the signs differ
+  const unsigned long long S = X + ((t ^ (unsigned long long)neg) - (unsigned long long)neg);
+  const unsigned int sh = (unsigned int)(S >> 32);
+  if (sh == 0u) return add_hw(a, b);
+  const unsigned int lz = (unsigned int)__clz((int)sh);
+  const unsigned int mh = __funnelshift_l((unsigned int)S, sh, lz), ml = (unsigned int)S << lz;
+  const unsigned int rl = __funnelshift_r(ml, mh, 11), rh = mh >> 11;
+  const unsigned int up = ((ml & 0x7ffu) + 0x3ffu + (rl & 1u)) >> 11;
+  const unsigned long long r =
+      (((unsigned long long)((xh & 0x80000000u) + ((ex - lz) << 20) + rh) << 32) | rl) + up;
+  return __longlong_as_double((long long)r);
+}
+
 // 1.0 - a, round to nearest even, on the integer pipe for 0 < a <= 1 (a particle's weight); the
 // rest takes the hardware subtraction.  With a in units of 2^-64 (truncated, and `rest` when bits were
 // lost: then a < 2^-11), R = 2^64 - a is exact, its leading 53 bits are the significand and the bits

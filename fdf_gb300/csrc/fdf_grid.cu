@@ -91,35 +91,39 @@ __global__ void k_build_planes(const double *__restrict__ coor, GridDims g, doub
 // The corner field (fdf_corner.cuh), one thread per node.  With cell_start non-null, nodes none of
 // whose adjacent cells holds a particle are skipped: the corner field is an intermediate of the
 // interpolation and only those nodes are ever read.
+// Bound by FP64 adds, 21 a node: of each component's seven two go to the integer pipe (masks 0x88: the
+// fourth and the eighth cell's), which then takes as long.  Per step 178 -> 132 us for 4.2M cells with 1M
+// particles, 628 -> 465 us for 14M with 16M (one component zero); with four to ten of the 21 there
+// 138/491, 137/448, 147/459, 157/489 us.  The lanes of a row's ends take the same path as the others, the
+// occupancy test reads a row's two cells at once and every index has 32 bits: with the former per-cell
+// branches six integer additions gained nothing (175 us).
 // AOS: the output is [Nn][3] instead of [3][Nn] (for the host).
 template <bool AOS>
 __global__ void k_center_to_corner(const double *__restrict__ ucat, GridDims g, double *__restrict__ corner,
                                    const unsigned int *__restrict__ cell_start, unsigned long long *nodes_done) {
-  long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  bool work = q < g.Nn;
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const bool work = q < g.Nn;
+  int i = 0, j = 0, k = 0;
+  if (work) node_ijk(g, (unsigned int)q, i, j, k);
   if (cell_start) {
-    // count the nodes this step computes (for the roofline bytes)
+    // count the nodes this step computes (for the roofline bytes); the cells of a row are neighbours in
+    // cell_start, so a row's are empty where nothing starts between the first and the one after the last
     bool need = false;
     if (work) {
-      int i0, j0, k0;
-      node_ijk(g, (unsigned int)q, i0, j0, k0);
-      for (int dk = -1; dk <= 0 && !need; ++dk)
-        for (int dj = -1; dj <= 0 && !need; ++dj)
-          for (int di = -1; di <= 0 && !need; ++di) {
-            int ck = k0 + dk, cj = j0 + dj, ci = i0 + di;
-            if (ci < 0 || ci >= g.IM || cj < 0 || cj >= g.JM || ck < 0 || ck >= g.KM) continue;
-            long long c = ((long long)ck * g.JM + cj) * g.IM + ci;
-            need = __ldg(cell_start + c + 1) > __ldg(cell_start + c);
-          }
+      const unsigned int i0 = max(i - 1, 0), i1 = min(i, g.IM - 1) + 1;
+      const unsigned int j0 = max(j - 1, 0), j1 = min(j, g.JM - 1), k0 = max(k - 1, 0), k1 = min(k, g.KM - 1);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const unsigned int row = (((e & 2) ? k1 : k0) * g.JM + ((e & 1) ? j1 : j0)) * g.IM;
+        need |= __ldg(cell_start + row + i1) > __ldg(cell_start + row + i0);
+      }
     }
     if (nodes_done) block_add_u64(need ? 1ull : 0ull, nodes_done);
     if (!need) return;
   }
   if (!work) return;
-  int i, j, k;
-  node_ijk(g, (unsigned int)q, i, j, k);
   double ox, oy, oz;
-  fdfx::corner_value(ucat, g, i, j, k, ox, oy, oz);
+  fdfx::corner_value<0x88, 0x88, 0x88>(ucat, g, i, j, k, ox, oy, oz);
   if (AOS) {
     corner[3 * q] = ox; corner[3 * q + 1] = oy; corner[3 * q + 2] = oz;
   } else {

@@ -5,6 +5,8 @@
 #include "fdf_exact.cuh"
 #include "fdf_corner.cuh"
 
+#include <algorithm>
+
 namespace {
 
 using fdfx::add;
@@ -13,7 +15,7 @@ using fdfx::mul;
 
 // ComputeTrilinearWeights (interpolation.c:839-864) and TrilinearInterpolation_Vector (:957-1042): the
 // velocity from the eight corner values value(c, x, y, z), c in bit order (i, j, k).
-template <typename Value>
+template <bool INT, typename Value>
 __device__ __forceinline__ void trilinear(double a1, double a2, double a3, Value value, double &ux, double &uy,
                                           double &uz) {
   a1 = fdfx::clamp01(a1);
@@ -23,8 +25,9 @@ __device__ __forceinline__ void trilinear(double a1, double a2, double a3, Value
   // w[c] = (x*y)*z as the reference evaluates it; the four (x*y) pair products are shared
   // The 36 products run on the integer pipe (fdfx::mul_int, the same bits as the FP64
   // multiply) and the sums on the FP64 pipe, so both pipes work at once.  Moving products back to
-  // the FP64 pipe (3 to 12 of them) is no faster: 4.64 to 5.28 against 4.66 ms for 64M particles.
-  auto wmul = [](double x, double y) { return fdfx::mul_int(x, y); };
+  // the FP64 pipe (3 to 12 of them) is no faster: 4.64 to 5.28 against 4.66 ms for 64M particles.  (Few
+  // particles: INT false, k_gather_interp.)
+  auto wmul = [](double x, double y) { return INT ? fdfx::mul_int(x, y) : mul(x, y); };
   const double p00 = wmul(oa1, oa2), p10 = wmul(a1, oa2), p01 = wmul(oa1, a2), p11 = wmul(a1, a2);
   double w[8];
   w[0] = wmul(p00, oa3); w[1] = wmul(p10, oa3); w[2] = wmul(p01, oa3); w[3] = wmul(p11, oa3);
@@ -72,8 +75,12 @@ __global__ void __launch_bounds__(256) k_pack(SwarmBuf b, const DevCounters *cnt
 // so resident warps beat the spills of 32 registers (64M particles 4.66 ms; 4.94 at 1536 threads, 5.0 at
 // 1280, 5.5 at the compiler's choice of 48 registers).
 // REC: the particles come from k_pack's records (mode GATHER_INTERP).
-template <bool REC>
-__global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf dst, GridDims g,
+// FEW: up to GATHER_FEW particles, about two and a half warps per scheduler, each warp's own chain is the time,
+// and the FP64 pipe's products and 128 registers make it shorter: 10k particles 11.0 -> 6.2 us, 30k 14.0 -> 12.2;
+// 100k 20.9 against 23, 1M 93 against 125, so not above.
+constexpr int GATHER_FEW = 3 << 14;
+template <bool REC, bool FEW>
+__global__ void __launch_bounds__(FEW ? 64 : 256, 8) k_gather_interp(SwarmBuf src, SwarmBuf dst, GridDims g,
                                                        const double *__restrict__ corner,
                                                        const unsigned int *__restrict__ perm,
                                                        const unsigned int *__restrict__ cell_start,
@@ -123,7 +130,7 @@ __global__ void __launch_bounds__(256, 8) k_gather_interp(SwarmBuf src, SwarmBuf
     cell_ijk(g, (unsigned int)cell, i, j, k);
     const long long mx = g.IM + 1, my = g.JM + 1;
     const double *at = corner + (((long long)k * my + j) * mx + i);
-    trilinear(a1, a2, a3, [&](int c, double &vx, double &vy, double &vz) {
+    trilinear<!FEW>(a1, a2, a3, [&](int c, double &vx, double &vy, double &vz) {
       const long long off = (c & 1) + ((c & 2) ? mx : 0) + ((c & 4) ? mx * my : 0);
       vx = __ldg(at + off); vy = __ldg(at + g.Nn + off); vz = __ldg(at + 2 * g.Nn + off);
     }, ux, uy, uz);
@@ -144,7 +151,7 @@ __global__ void __launch_bounds__(128) k_interp_points(const long long *__restri
   double ux = 0.0, uy = 0.0, uz = 0.0;
   if (i >= 0 && i < g.IM && j >= 0 && j < g.JM && k >= 0 && k < g.KM) {
     const long long mx = g.IM + 1, my = g.JM + 1;
-    trilinear(weight[3 * (size_t)p], weight[3 * (size_t)p + 1], weight[3 * (size_t)p + 2],
+    trilinear<true>(weight[3 * (size_t)p], weight[3 * (size_t)p + 1], weight[3 * (size_t)p + 2],
               [&](int c, double &vx, double &vy, double &vz) {
                 const int ni = (int)i + (c & 1), nj = (int)j + ((c >> 1) & 1), nk = (int)k + (c >> 2);
                 if (DIRECT) {
@@ -434,7 +441,11 @@ void launch_gather_interp(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, G
   int th = 256;
   int blocks = (n_cap + th - 1) / th;
   if (blocks == 0) blocks = 1;
-  k_gather_interp<false><<<blocks, th, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode, nullptr);
+  if (n_cap <= GATHER_FEW)
+    k_gather_interp<false, true><<<std::max((n_cap + 63) / 64, 1), 64, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt,
+                                                                              mode, nullptr);
+  else
+    k_gather_interp<false, false><<<blocks, th, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, mode, nullptr);
 }
 
 void launch_gather_interp_packed(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const double *corner,
@@ -443,7 +454,7 @@ void launch_gather_interp_packed(const SwarmBuf &src, const SwarmBuf &dst, int n
   const unsigned int blocks = n_cap > 0 ? (unsigned int)((n_cap + 255) / 256) : 1u;
   ulonglong2 *r = static_cast<ulonglong2 *>(rec);
   k_pack<<<blocks, 256, 0, s>>>(src, cnt, r);
-  k_gather_interp<true><<<blocks, 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, GATHER_INTERP, r);
+  k_gather_interp<true, false><<<blocks, 256, 0, s>>>(src, dst, g, corner, perm, cell_start, cnt, GATHER_INTERP, r);
 }
 
 void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int *cell_start, double volume, double *count,

@@ -279,20 +279,19 @@ MLP_FLOPS = 2 * (3 * 128 + 128 * 128 + 128 * 128 + 128 * 3)   # per particle, on
 # DRAM bytes (read + write) per launch of a stage's kernels, measured by ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum, one pass) on this workload at full size, with
 # the units the stage processed then: live particles, or guessed particles for the network and
-# the walk from the guess.  The precision forms' sort stage: scan and slot scatter as captured
-# with the PID-ordered sort, plus the ordering kernel captured since it orders by previous slot
-# (0.364 GB instead of 1.02 GB per launch).
+# the walk from the guess.  The FP32 walk and the plain form's kernels as captured before their rows were
+# swizzled and their chains changed: the same arrays read and written.
 TRAFFIC = {
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "advect_locate"): (7.757e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "learned_guess"): (0.596e9, "guesses", 12.92e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "guess_walk"): (2.063e9, "guesses", 12.92e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "sort_by_cell"): (1.213e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "gather_interpolate"): (7.906e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "deposit"): (1.345e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "advect_locate"): (7.740e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "learned_guess"): (0.598e9, "guesses", 12.92e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "guess_walk"): (2.093e9, "guesses", 12.92e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "deposit"): (1.352e9, "particles", 63.81e6),
     ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "advect_locate"): (7.623e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "sort_by_cell"): (1.213e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "gather_interpolate"): (7.906e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "deposit"): (1.345e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
+    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "deposit"): (1.352e9, "particles", 63.81e6),
     ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "advect_locate"): (13.444e9, "particles", 63.81e6),
     ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "gather_interpolate"): (10.885e9, "particles", 63.81e6),
     ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "deposit"): (2.651e9, "particles", 63.81e6),
@@ -652,7 +651,8 @@ def fp32_errors_full(ctx, wl, steps: int, sample: int, nthreads: int) -> dict:
     return out
 
 
-FP64_OPS_C2C = 21      # 3 face sums, 9 products, 6 sums, 3 scalings per interior cell
+FP64_OPS_C2C = 14      # on the FP64 pipe, of 3 face sums, 9 products, 6 sums and 3 scalings per interior cell (7 products
+                       # run on the integer pipe)
 CLOCK_MAX_MHZ = 2070   # GB300 maximum SM clock
 
 
@@ -686,8 +686,7 @@ def time_contra2cart(ctx, wl, calls: int) -> dict:
     alg = 116 * n_int + 24 * Nn        # table 80 + ucat 24 + ucat32 12 per interior cell, face velocity per node
     hbm, peak_kind = peaks()
     gbs = alg / (ms / 1000.0) / 1e9
-    # the bound: GB300's FP64 pipe, two lanes per clock per SM (ncu: sm__pipe_fp64_cycles_active
-    # 83 % with 21 FP64 instructions per cell)
+    # the bound: GB300's FP64 pipe, two lanes per clock per SM, and the integer pipe beside it
     import torch
     sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     fp64_peak = 2.0 * sms * CLOCK_MAX_MHZ * 1e6 / 1e9

@@ -19,7 +19,7 @@
 #include <cuda_runtime.h>
 
 #define FDF_ROW 38            // doubles per plane-table row (36 plane values + thr + flag)
-#define FDF_ROW32 32          // floats per FP32 plane-table row: 128 B (c0 pair, thr32, slack, 6 x (n32, e32))
+#define FDF_ROW32 32          // floats per FP32 plane-table row: 128 B (c0 pair, the cell's margin, thr32 + slack, 6 x (n32, e32))
 #define FDF_MAX_TRAVERSAL 1000
 #define FDF_DISTANCE_THRESHOLD 1e-11
 #define FDF_INTERP_DIST_TOL 1e-14
@@ -141,9 +141,9 @@ __device__ __forceinline__ void node_ijk(const GridDims &g, unsigned int q, int 
 #ifndef FDF_LOC_MIN_BLOCKS
 #define FDF_LOC_MIN_BLOCKS (1024 / FDF_LOC_THREADS)
 #endif
-// Resident blocks per SM of the plain walk (its steps decided from the FP32 table; per
-// 64M-particle step 1024 resident threads take 7.6 ms against 8.6 ms at 768 and 8.4 ms at 1280
-// or 1536, where spills grow) and of the per-cell PID ordering (latency-bound: 2048 resident threads at 32 registers,
+// Resident blocks per SM of the plain walk with all its products on the FP64 pipe (1024 threads: 83 us
+// for 500k particles, 86 at 1280; one block more where two products of three leave that pipe, fdf_walk.cu)
+// and of the per-cell PID ordering (latency-bound: 2048 resident threads at 32 registers,
 // 1.59 -> 1.24 ms for the 64M-particle sort stage).
 #ifndef FDF_PLAIN_MIN_BLOCKS
 #define FDF_PLAIN_MIN_BLOCKS 8

@@ -147,8 +147,12 @@ __device__ __forceinline__ unsigned int settle_key32(bool lost, int cell, float2
 //                   walk's second cell, and finished by k_locate32_path (its key and
 //                   histogram entry are written there); a nearer one continues the reference
 //                   walk here.
-template <bool FIRST, bool FAR>
-__global__ void __launch_bounds__(FDF_LOC_THREADS, FDF_LOC_MIN_BLOCKS) k_locate32(SwarmBuf b, GridDims g, const float *__restrict__ table,
+//   DENSE: more slots than cells.  A warp's rows then mostly come from L1 and L2 and two more blocks an SM
+//          (56 registers, a few spilled) hide more of the walk than the spills cost: per step 64M particles
+//          in 14M cells 2.29 -> 2.20 ms, the learned form's first pass 2.32 -> 2.17, 16M in 4.2M cells
+//          0.518 -> 0.493; 6M in 14M cells 0.285 against 0.290 (four more: 2.47, 2.19, 0.554, 0.333).
+template <bool FIRST, bool FAR, bool DENSE>
+__global__ void __launch_bounds__(FDF_LOC_THREADS, FDF_LOC_MIN_BLOCKS + (DENSE ? 128 / FDF_LOC_THREADS : 0)) k_locate32(SwarmBuf b, GridDims g, const float *__restrict__ table,
                                                   const double *__restrict__ planes, float dt32, int advect,
                                                   int reset_first, const double *__restrict__ bbox,
                                                   const float *__restrict__ fbox, int drop_removed,
@@ -791,10 +795,13 @@ void launch_locate32(const SwarmBuf &b, int n_cap, GridDims g, const float *tabl
                                                 drop_removed, cnt, keys, rank, count, sentinel, pend, n_cap, far);
   };
   // without the advection the particles come from anywhere (the initial setup's corner start)
-  if (pending && advect) go(k_locate32<true, false>, pending, far_cells);
-  else if (pending) go(k_locate32<true, true>, pending, far_cells);
-  else if (advect) go(k_locate32<false, false>, nullptr, 0.f);
-  else go(k_locate32<false, true>, nullptr, 0.f);
+  const bool dense = n_cap > g.Nc;
+  if (pending && advect && dense) go(k_locate32<true, false, true>, pending, far_cells);
+  else if (pending && advect) go(k_locate32<true, false, false>, pending, far_cells);
+  else if (pending) go(k_locate32<true, true, false>, pending, far_cells);
+  else if (advect && dense) go(k_locate32<false, false, true>, nullptr, 0.f);
+  else if (advect) go(k_locate32<false, false, false>, nullptr, 0.f);
+  else go(k_locate32<false, true, false>, nullptr, 0.f);
 }
 
 void launch_compact_pending(const unsigned int *scan, int n_cap, unsigned int *list, DevCounters *cnt,

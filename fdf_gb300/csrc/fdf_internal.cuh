@@ -134,10 +134,9 @@ __device__ __forceinline__ void node_ijk(const GridDims &g, unsigned int q, int 
 #ifndef FDF_LOC_THREADS
 #define FDF_LOC_THREADS 64
 #endif
-// Resident blocks per SM the FP32 locate kernels are compiled for: 1024 threads leave 64 registers,
-// the most threads without a spill in the walk's loop (per 64M-particle step 2.30 ms; 2.45 at 1152
-// threads and 2.68 at 1280, whose spills go through the L1 data pipe that the row loads need; 2.66 at
-// 896, 2.90 at 768).
+// Resident blocks per SM the FP32 locate kernels are compiled for (k_locate32: two more in dense swarms):
+// 1024 threads leave 64 registers, the most threads without a spill in the walk's loop (at 896 2.66 ms per
+// 64M-particle step, at 768 2.90, against 2.30).
 #ifndef FDF_LOC_MIN_BLOCKS
 #define FDF_LOC_MIN_BLOCKS (1024 / FDF_LOC_THREADS)
 #endif

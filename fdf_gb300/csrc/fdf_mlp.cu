@@ -34,7 +34,9 @@ __device__ __forceinline__ float silu_grad(float z) {
 
 // Programmatic dependent launch: a kernel launched with launch_after may begin before the one ahead of
 // it on the stream has ended (once that one's blocks have all called let_next_start, or ended) and
-// calls await_previous before it touches anything the earlier kernels write.
+// calls await_previous before it touches anything the earlier kernels write.  What they write is not
+// constant for the whole of this kernel's life, so no pointer to it is `__restrict__`: that would allow
+// the loads to pass the wait or to take the read-only path.
 __device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>
@@ -174,11 +176,10 @@ __device__ __forceinline__ unsigned bf16x2(float lo, float hi) {
 }
 
 __global__ void __launch_bounds__(TT_THREADS, 1)
-    k_train_tc(const unsigned char *__restrict__ wimg, const float *__restrict__ params, const float *__restrict__ xs,
+    k_train_tc(const unsigned char *wimg, const float *params, const float *__restrict__ xs,
                const float *__restrict__ ts, long long n_samples, unsigned long long seed, long long step,
-               int hashed, int B, float sx, float sy, float sz, float *__restrict__ part,
-               float *__restrict__ loss_part, unsigned int *__restrict__ err, unsigned long long wait_limit,
-               int stall_test) {
+               int hashed, int B, float sx, float sy, float sz, float *part, float *loss_part, unsigned int *err,
+               unsigned long long wait_limit, int stall_test) {
   using namespace fdftc;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -478,10 +479,9 @@ __global__ void __launch_bounds__(TT_THREADS, 1)
 
 // grads = the tiles' partials added in tile order; with adam, the Adam step (as k_adam) on the
 // FP32 parameters and their bfloat16 image rewritten for the next step.
-__global__ void k_train_update(const float *__restrict__ part, int tiles, const float *__restrict__ loss_part,
-                               float *__restrict__ params, float *__restrict__ grads, float *__restrict__ m,
-                               float *__restrict__ v, unsigned char *__restrict__ wimg, float *__restrict__ loss_out,
-                               int adam, float lr, float c1, float c2) {
+__global__ void k_train_update(const float *part, int tiles, const float *loss_part, float *params, float *grads,
+                               float *m, float *v, unsigned char *wimg, float *loss_out, int adam, float lr, float c1,
+                               float c2) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   await_previous();
   let_next_start();
@@ -491,15 +491,17 @@ __global__ void k_train_update(const float *__restrict__ part, int tiles, const 
     *loss_out = l;
   }
   if (q >= MLP_NPARAM) return;
+  float m0 = 0.f, v0 = 0.f, w0 = 0.f;   // loaded beside the partials
+  if (adam) { m0 = m[q]; v0 = v[q]; w0 = params[q]; }
   float g = 0.f;
   for (int t = 0; t < tiles; ++t) g += part[(long long)t * MLP_PART_STRIDE + q];
   grads[q] = g;
   if (!adam) return;
-  const float mq = 0.9f * m[q] + 0.1f * g;
-  const float vq = 0.999f * v[q] + 0.001f * g * g;
+  const float mq = 0.9f * m0 + 0.1f * g;
+  const float vq = 0.999f * v0 + 0.001f * g * g;
   m[q] = mq;
   v[q] = vq;
-  const float w = params[q] - lr * (mq / c1) / (sqrtf(vq / c2) + 1e-8f);
+  const float w = w0 - lr * (mq / c1) / (sqrtf(vq / c2) + 1e-8f);
   params[q] = w;
   const __nv_bfloat16 wb = __float2bfloat16_rn(w);
   const unsigned short bits = *reinterpret_cast<const unsigned short *>(&wb);

@@ -314,6 +314,87 @@ __global__ void __launch_bounds__(DEP_WARPS * 32, MOM ? 4 : 8) k_deposit(SwarmBu
   face(node && i < IM && j < JM, k > 0, c - (long long)IM * JM, b.a3, fk, mk, nfk, c);
 }
 
+// The same sums with a node's four chains -- the cell's P and its three faces -- in four blocks (blockIdx.y),
+// for grids whose nodes do not fill the chip: one thread then waits for one chain instead of four in a
+// row, with four particles' loads and products under way before their adds.  Products on the integer
+// pipe for the volume, on the FP64 pipe for the momentum, whose 24 a particle would lengthen the chain.
+// 18k nodes (20 x 20 x 40 cells), 60 particles per cell: 73 us against 166 in one chain after another, with the
+// momentum 213 against 325; 71k nodes, 30 per cell 105 against 123; 274k nodes, 18 per cell 195 against 227.
+template <bool MOM>
+__global__ void __launch_bounds__(DEP_WARPS * 32, MOM ? 4 : 8) k_deposit_apart(SwarmBuf b, GridDims g,
+                                                                              const unsigned int *__restrict__ cs,
+                                                                              double third, double *__restrict__ count,
+                                                                              double *__restrict__ avg,
+                                                                              double *__restrict__ fi,
+                                                                              double *__restrict__ fj,
+                                                                              double *__restrict__ fk,
+                                                                              double *__restrict__ mi,
+                                                                              double *__restrict__ mj,
+                                                                              double *__restrict__ mk) {
+  constexpr int V = MOM ? 4 : 1, CH = 4;
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (q >= g.Nn) return;
+  const int IM = g.IM, JM = g.JM, KM = g.KM, f = blockIdx.y;   // f: the face's direction, 3 the cell
+  int i, j, k;
+  node_ijk(g, (unsigned int)q, i, j, k);
+  const long long c = ((long long)k * JM + j) * IM + i;
+  unsigned int s0 = 0u, s1 = 0u;
+  if (i < IM && j < JM && k < KM) { s0 = __ldg(cs + c); s1 = __ldg(cs + c + 1); }
+  if (f == 3) {
+    double sum = 0.0;
+    for (unsigned int s = s0; s < s1; s += CH) {
+      double P[CH];
+#pragma unroll
+      for (int e = 0; e < CH; ++e) P[e] = s + e < s1 ? __ldg(b.P + s + e) : 0.0;
+#pragma unroll
+      for (int e = 0; e < CH; ++e)
+        if (s + e < s1) sum = add(sum, P[e]);
+    }
+    const unsigned int ncell = s1 - s0;
+    count[q] = fdfx::u32_to_double(ncell);
+    avg[q] = ncell > 0 ? fdfx::div_count(sum, ncell) : 0.0;
+    return;
+  }
+  if ((f != 0 && i >= IM) || (f != 1 && j >= JM) || (f != 2 && k >= KM)) return;   // no such face
+  const long long lower = c - (f == 0 ? 1LL : f == 1 ? (long long)IM : (long long)IM * JM);
+  unsigned int l0 = 0u, l1 = 0u;
+  if ((f == 0 ? i : f == 1 ? j : k) > 0) { l0 = __ldg(cs + lower); l1 = __ldg(cs + lower + 1); }
+  const double *__restrict__ wgt = f == 0 ? b.a1 : f == 1 ? b.a2 : b.a3;
+  const unsigned int nl = l1 - l0, T = nl + (s1 - s0);
+  auto product = [](double x, double y) { return MOM ? mul(x, y) : fdfx::mul_int(x, y); };
+  double acc[V];
+#pragma unroll
+  for (int m = 0; m < V; ++m) acc[m] = 0.0;
+  for (unsigned int t = 0; t < T; t += CH) {
+    double x[CH][V];
+#pragma unroll
+    for (int e = 0; e < CH; ++e) {
+      const unsigned int s = t + e < nl ? l0 + (t + e) : s0 + (t + e - nl);
+      const bool in = t + e < T;
+      const double a = in ? __ldg(wgt + s) : 0.0;
+      x[e][0] = product(t + e < nl ? a : sub(1.0, a), third);
+      if (MOM) {
+        x[e][V - 3] = product(x[e][0], in ? __ldg(b.u + s) : 0.0);
+        x[e][V - 2] = product(x[e][0], in ? __ldg(b.v + s) : 0.0);
+        x[e][V - 1] = product(x[e][0], in ? __ldg(b.w + s) : 0.0);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < CH; ++e)
+      if (t + e < T) {
+#pragma unroll
+        for (int m = 0; m < V; ++m) acc[m] = add(acc[m], x[e][m]);
+      }
+  }
+  const long long at = f == 0 ? ((long long)k * JM + j) * (IM + 1) + i : f == 1 ? ((long long)k * (JM + 1) + j) * IM + i : c;
+  (f == 0 ? fi : f == 1 ? fj : fk)[at] = acc[0];
+  if (MOM) {
+    const long long nf = f == 0 ? (IM + 1LL) * JM * KM : f == 1 ? IM * (JM + 1LL) * KM : (long long)IM * JM * (KM + 1LL);
+    double *mom = f == 0 ? mi : f == 1 ? mj : mk;
+    mom[at] = acc[V - 3]; mom[nf + at] = acc[V - 2]; mom[2 * nf + at] = acc[V - 1];
+  }
+}
+
 // Slot t of dst takes slot a + t of src for t < b - a, and slot c + (t - (b - a)) after that: the
 // held particles of a k-slab ([a, b) in the cell-sorted order) followed by those without a cell
 // ([c, n)); every field of both forms moves.
@@ -466,8 +547,18 @@ void launch_deposit(const SwarmBuf &b, int n_cap, GridDims g, const unsigned int
   // Above five particles per cell most warps' ranges exceed DEP_CAP, and the staging's shared memory
   // only takes from the L1 cache (27 per cell, 32M particles: 1.25 ms staged, 1.09 without; 4.5 per
   // cell, 64M: 2.20 staged, 2.85 without).  The capacity stands for the count, which only the device knows.
-  if (mi) k_deposit<true, false><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
-  else if (n_cap <= 5 * g.Nc)
+  const bool dense = n_cap > 5 * g.Nc;
+  // The chains apart: with 18k nodes faster at every density (one and 4.9 per cell: 16.4 and 22.0 us against
+  // 20.8 and 35.3 staged, momentum 22.6 and 38.1 against 30.7 and 57.6), with 71k nodes staged (23.1 and 29.7
+  // at one and three per cell against 22.3 and 30.1) or with the momentum (36.2 and 97 at one and eight against
+  // 38.1 and 119) no longer.  Without the staging up to half a million nodes: 274k nodes 111 against 127 us at
+  // eight per cell, 195 against 229 at 18; 545k nodes 207 against 207, 365 against 376; 1.2M 437 against 417.
+  const bool apart = g.Nn <= (1 << 15) || (!mi && dense && g.Nn <= (1 << 19));
+  const dim3 four(blocks, 4);
+  if (apart && mi) k_deposit_apart<true><<<four, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
+  else if (apart) k_deposit_apart<false><<<four, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
+  else if (mi) k_deposit<true, false><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
+  else if (!dense)
     k_deposit<false, true><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
   else k_deposit<false, false><<<blocks, th, 0, s>>>(b, g, cell_start, third, count, avg, fi, fj, fk, mi, mj, mk);
 }

@@ -643,6 +643,7 @@ int read_info(FdfContext *ctx, FdfStepInfo *info) {
   if (c.err & ERRBIT_DEGENERATE)
     return fail(ctx, FDF_ERR_USER, "Degenerate plane detected (normal vector is near zero).");
   if (c.err & ERRBIT_TC_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "learned locator: tensor-core wait timed out");
+  if (c.err & ERRBIT_SORT_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "sort of the LOST particles: wait timed out");
   return FDF_SUCCESS;
 }
 
@@ -717,7 +718,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
   // the plain form orders each cell by PID (the oracle's summation order); the precision forms
   // keep each cell's particles in their previous order (no gather of the PIDs)
   ctx->launches += launch_order_segments(ctx->cell_start, (int)g.Nc, f32 ? nullptr : src.pid, ctx->perm,
-                                         drop ? nullptr : ctx->rank, ctx->cap, s);
+                                         drop ? nullptr : ctx->rank, ctx->cap, ctx->cnt, ctx->num_sms, s);
   size_t e2 = prof ? record_event(ctx, s) : 0;
   if (!locate_only) CU(cudaStreamWaitEvent(s, ctx->ev_corner, 0));
   size_t e3 = prof ? record_event(ctx, s) : 0;
@@ -792,8 +793,8 @@ int resort(FdfContext *ctx, int remove_lost, int remove_oob, int64_t *removed_lo
                      ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, s);
   ctx->launches += 3 + scan_histogram(ctx->hist, ctx->cell_start, g.Nc + 2, ctx->scan_sums, s);   // keys, slots, gather
   launch_scatter_slots(ctx->keys, ctx->rank, ctx->cap, ctx->cnt, ctx->sentinel, 1, ctx->cell_start, ctx->perm, s);
-  ctx->launches += launch_order_segments(ctx->cell_start, (int)g.Nc, f32 ? nullptr : src.pid, ctx->perm, ctx->rank,
-                                         ctx->cap, s);
+  ctx->launches += launch_order_segments(ctx->cell_start, (int)g.Nc, f32 ? nullptr : src.pid, ctx->perm,
+                                         ctx->rank, ctx->cap, ctx->cnt, ctx->num_sms, s);
   if (f32)
     launch_gather_interp32(src, dst, ctx->cap, g, ctx->corner32, ctx->perm, ctx->cell_start, ctx->cnt, s, GATHER_COPY);
   else
@@ -807,6 +808,7 @@ int resort(FdfContext *ctx, int remove_lost, int remove_oob, int64_t *removed_lo
   CU(cudaStreamSynchronize(s));
   if (removed_lost) *removed_lost = (int64_t)c.removed_lost;
   if (removed_oob) *removed_oob = (int64_t)c.removed_oob;
+  if (c.err & ERRBIT_SORT_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "sort of the LOST particles: wait timed out");
   return FDF_SUCCESS;
 }
 

@@ -34,7 +34,7 @@ enum { ST_NEEDS_LOCATION = 0, ST_ACTIVE_AND_LOCATED = 1, ST_MIGRATING_OUT = 2, S
        ST_UNINITIALIZED = 4 };
 
 // Device error word bits.
-enum { ERRBIT_DEGENERATE = 1u, ERRBIT_TC_TIMEOUT = 4u };
+enum { ERRBIT_DEGENERATE = 1u, ERRBIT_TC_TIMEOUT = 4u, ERRBIT_SORT_TIMEOUT = 8u };
 
 // The walk kernels' block flushes go to one of FDF_CNT_STRIPES rows (by block index), so that
 // they spread over the L2 slices instead of queueing on one line; the slot scatter's last block
@@ -42,6 +42,8 @@ enum { ERRBIT_DEGENERATE = 1u, ERRBIT_TC_TIMEOUT = 4u };
 #define FDF_CNT_STRIPES 512
 enum { CNT_LOST = 0, CNT_OOB = 1, CNT_EVALS = 2, CNT_EVALS_TOTAL = 3, CNT_LOST_TOTAL = 4, CNT_FB = 5,
        CNT_SLOTS = 8 };
+
+constexpr int LOST_BARRIERS = 20;   // merges of 2^29 slots from runs of 2^11, and two more
 
 // Counters kept on the device so that a step needs no host round trip.
 struct DevCounters {
@@ -67,6 +69,8 @@ struct DevCounters {
   unsigned long long fallback_evals_total;   // (unused: zero)
   // pending block flushes (fold_counts); rows of 64 bytes
   alignas(64) unsigned long long stripes[FDF_CNT_STRIPES][CNT_SLOTS];
+  // blocks that came to each barrier of the LOST particles' merges, and to their end; zero between launches
+  unsigned int lost_arrived[LOST_BARRIERS + 1];
 };
 // The counters without the flush rows (what the host reads back).
 #define DEVCOUNTERS_HEAD offsetof(DevCounters, stripes)
@@ -233,9 +237,9 @@ void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, in
                           unsigned int sentinel, int keep_lost, const unsigned int *cell_start, unsigned int *perm,
                           cudaStream_t s);
 // Orders every cell's slots by (PID, previous slot), or by previous slot when pid is null; with
-// lost_scratch [n_cap], also the LOST particles' bucket ncells.  Returns the kernels launched.
+// lost_scratch [n_cap], also the LOST particles' bucket ncells (cnt: its barriers).  Returns the kernels launched.
 int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
-                           unsigned int *lost_scratch, int n_cap, cudaStream_t s);
+                          unsigned int *lost_scratch, int n_cap, DevCounters *cnt, int num_sms, cudaStream_t s);
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
                           unsigned int *cell_start, unsigned int *rank, unsigned int *cursor, unsigned int *sums,
                           cudaStream_t s);

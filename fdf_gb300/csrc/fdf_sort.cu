@@ -396,82 +396,91 @@ __global__ void __launch_bounds__(256, FDF_ORDER_MIN_BLOCKS) k_order_segments(co
 // The LOST particles that the initial setup and the staged calls keep: one bucket, which may hold a
 // few percent of the swarm, ordered like the cells' slots but by the whole GPU.  Chunks of
 // LOST_CHUNK entries are sorted in shared memory, then neighbouring runs are merged, twice as long
-// each time, between perm and `other`: every entry finds its rank in the partner run by binary
-// search.  The host knows only the swarm's capacity, so the merges it cannot rule out are launched
-// and return at once (1.5 us each).  (A single thread's insertion sort took 0.40 s for the 20,000
-// LOST of 1M particles on the sinusoidal 64x64x1024 grid, 0.94 s for the 78,000 of 6M on 96x96x1536.)
+// each time, between perm and `other` (both indexed like perm): every entry finds its rank in the
+// partner run by binary search.  Only the device knows how many there are, so the merges are one
+// launch with a barrier of the grid between them (cooperative: one block per SM, all resident): with none
+// LOST it costs 2 us at any capacity, where a launch for each merge that the capacity allowed took
+// 2.5 us each (removing the LOST of a million slots 153 us against 117 without them).  (A single thread's
+// insertion sort took 0.40 s for the 20,000 LOST of 1M particles on the sinusoidal 64x64x1024 grid,
+// 0.94 s for the 78,000 of 6M on 96x96x1536.)
 constexpr int LOST_CHUNK = 2048, LOST_THREADS = 1024;
 
+// Polls of a barrier before it is given up (seconds; the longest merge, of 2^29 entries, takes a tenth).
+constexpr unsigned int LOST_WAIT_LIMIT = 1u << 24;
+
+// Barrier number m of this launch: false (in every thread of the block) when the wait ran out.
+__device__ __forceinline__ bool lost_barrier(unsigned int *arrived, int m) {
+  __shared__ unsigned int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived + m, 1u);
+    unsigned int it = 0;
+    while (*reinterpret_cast<volatile unsigned int *>(arrived + m) < gridDim.x && it < LOST_WAIT_LIMIT) ++it;
+    ok = it < LOST_WAIT_LIMIT ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0u;
+}
+
 template <bool PID>
-__global__ void __launch_bounds__(LOST_THREADS) k_lost_chunks(const unsigned int *__restrict__ bucket,
-                                                             const long long *__restrict__ pid,
-                                                             unsigned int *__restrict__ perm) {
+__global__ void __launch_bounds__(LOST_THREADS, 1) k_order_lost(const unsigned int *__restrict__ bucket,
+                                                              const long long *__restrict__ pid, unsigned int *perm,
+                                                              unsigned int *other, DevCounters *cnt) {
   using Key = SlotKey<PID>;
   __shared__ Key item[LOST_CHUNK];
   const unsigned int s0 = bucket[0], L = bucket[1] - s0;
+  if (L <= 1u) return;
+  int merges = 0;
+  for (unsigned long long r = LOST_CHUNK; r < L; r <<= 1) ++merges;
+  unsigned int *to = merges & 1 ? other : perm, *from = perm;   // the last merge ends in perm
   for (unsigned int c0 = blockIdx.x * LOST_CHUNK; c0 < L; c0 += gridDim.x * LOST_CHUNK) {
     const unsigned int n = min(L - c0, (unsigned int)LOST_CHUNK);
-    unsigned int *run = perm + s0 + c0;
-    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) item[e] = slot_key<PID>(run[e], pid);
+    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) item[e] = slot_key<PID>(perm[s0 + c0 + e], pid);
     __syncthreads();
     block_bitonic(n, [&](unsigned int i) { return item[i]; }, [&](unsigned int i, const Key &v) { item[i] = v; });
-    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) run[e] = item[e].slot;
+    for (unsigned int e = threadIdx.x; e < n; e += blockDim.x) to[s0 + c0 + e] = item[e].slot;
     __syncthreads();
   }
-}
-
-// Merges runs of `run` entries pairwise from `from` to `to` (both indexed like perm) while the
-// bucket holds more than one; last: copies the result back to `to` = perm when the merges made (one
-// per doubling of LOST_CHUNK below the bucket's length) left it in the other array.
-template <bool PID>
-__global__ void __launch_bounds__(256) k_lost_merge(const unsigned int *__restrict__ bucket,
-                                                   const long long *__restrict__ pid, unsigned int run,
-                                                   const unsigned int *__restrict__ from,
-                                                   unsigned int *__restrict__ to, int last) {
-  const unsigned int s0 = bucket[0], L = bucket[1] - s0;
+  if (merges == 0) return;
   const unsigned int stride = gridDim.x * blockDim.x;
-  if (last) {
-    int merges = 0;
-    for (unsigned long long r = LOST_CHUNK; r < L; r <<= 1) ++merges;
-    if (merges & 1)
-      for (unsigned int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += stride) to[s0 + p] = from[s0 + p];
-    return;
-  }
-  if (run >= L) return;
-  for (unsigned int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += stride) {
-    const unsigned int v = from[s0 + p];
-    const SlotKey<PID> k = slot_key<PID>(v, pid);
-    const unsigned int own = p / run * run, pair = own / (2 * run) * (2 * run);
-    unsigned int lo = own == pair ? min(own + run, L) : pair, base = lo;
-    unsigned int hi = own == pair ? min(lo + run, L) : own;
-    while (lo < hi) {   // the partner's entries before k: keys are distinct (slots differ)
-      const unsigned int mid = lo + (hi - lo) / 2;
-      if (k.after(slot_key<PID>(from[s0 + mid], pid))) lo = mid + 1;
-      else hi = mid;
+  unsigned int run = LOST_CHUNK;
+  for (int m = 0; m < merges; ++m, run <<= 1) {
+    if (!lost_barrier(cnt->lost_arrived, m)) {
+      if (threadIdx.x == 0) atomicOr(&cnt->err, (unsigned int)ERRBIT_SORT_TIMEOUT);
+      return;
     }
-    to[s0 + pair + (p - own) + (lo - base)] = v;
-  }
-}
-
-// Returns the number of kernels launched.
-template <bool PID>
-int order_lost(const unsigned int *bucket, const long long *pid, unsigned int *perm, unsigned int *other, int n_cap,
-                cudaStream_t s) {
-  const long long chunks = ((long long)n_cap + LOST_CHUNK - 1) / LOST_CHUNK;
-  const unsigned int blocks = (unsigned int)std::min<long long>(std::max<long long>(chunks, 1), 304);
-  k_lost_chunks<PID><<<blocks, LOST_THREADS, 0, s>>>(bucket, pid, perm);
-  if (n_cap <= LOST_CHUNK) return 1;
-  int launched = 2;
-  const unsigned int *from = perm;
-  unsigned int *to = other;
-  for (long long run = LOST_CHUNK; run < n_cap; run *= 2) {
-    k_lost_merge<PID><<<4 * blocks, 256, 0, s>>>(bucket, pid, (unsigned int)run, from, to, 0);
     from = to;
     to = from == perm ? other : perm;
-    ++launched;
+    for (unsigned int p = blockIdx.x * blockDim.x + threadIdx.x; p < L; p += stride) {
+      const unsigned int v = from[s0 + p];
+      const Key k = slot_key<PID>(v, pid);
+      const unsigned int own = p / run * run, pair = own / (2 * run) * (2 * run);
+      unsigned int lo = own == pair ? min(own + run, L) : pair, base = lo;
+      unsigned int hi = own == pair ? min(lo + run, L) : own;
+      while (lo < hi) {   // the partner's entries before k: keys are distinct (slots differ)
+        const unsigned int mid = lo + (hi - lo) / 2;
+        if (k.after(slot_key<PID>(from[s0 + mid], pid))) lo = mid + 1;
+        else hi = mid;
+      }
+      to[s0 + pair + (p - own) + (lo - base)] = v;
+    }
   }
-  k_lost_merge<PID><<<4 * blocks, 256, 0, s>>>(bucket, pid, 0u, other, perm, 1);
-  return launched;
+  // the last block to come here has every block past every barrier: it clears their counts
+  if (threadIdx.x == 0 && atomicAdd(cnt->lost_arrived + LOST_BARRIERS, 1u) == gridDim.x - 1) {
+    for (int m = 0; m <= LOST_BARRIERS; ++m) cnt->lost_arrived[m] = 0u;
+  }
+}
+
+template <bool PID>
+void order_lost(const unsigned int *bucket, const long long *pid, unsigned int *perm, unsigned int *other, int n_cap,
+                DevCounters *cnt, int num_sms, cudaStream_t s) {
+  const long long chunks = ((long long)n_cap + LOST_CHUNK - 1) / LOST_CHUNK;
+  const unsigned int blocks = (unsigned int)std::min<long long>(std::max<long long>(chunks, 1), num_sms);
+  void *args[] = {&bucket, &pid, &perm, &other, &cnt};
+  cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_order_lost<PID>), dim3(blocks), dim3(LOST_THREADS), args, 0,
+                              s);   // errors through cudaGetLastError
 }
 
 // count[cell[s]] += 1 for 0 <= cell[s] < ncells (warp-aggregated integer atomics)
@@ -681,13 +690,14 @@ void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, in
 }
 
 int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
-                           unsigned int *lost_scratch, int n_cap, cudaStream_t s) {
+                          unsigned int *lost_scratch, int n_cap, DevCounters *cnt, int num_sms, cudaStream_t s) {
   const int th = 256, blocks = (ncells + th - 1) / th;
   if (pid) k_order_segments<true><<<blocks, th, 0, s>>>(cell_start, ncells, pid, perm);
   else k_order_segments<false><<<blocks, th, 0, s>>>(cell_start, ncells, nullptr, perm);
   if (!lost_scratch) return 1;
-  return 1 + (pid ? order_lost<true>(cell_start + ncells, pid, perm, lost_scratch, n_cap, s)
-                  : order_lost<false>(cell_start + ncells, nullptr, perm, lost_scratch, n_cap, s));
+  if (pid) order_lost<true>(cell_start + ncells, pid, perm, lost_scratch, n_cap, cnt, num_sms, s);
+  else order_lost<false>(cell_start + ncells, nullptr, perm, lost_scratch, n_cap, cnt, num_sms, s);
+  return 2;
 }
 
 // Stable counting sort of particle slots by cell id, on caller-provided scratch: sums
@@ -714,5 +724,5 @@ void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsign
   exclusive_scan_u32(cell_start, ncells + 1, sums, s);
   if (rank) k_cell_place<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank, perm);
   else k_cell_slots<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start, cursor, perm);
-  launch_order_segments(cell_start, (int)ncells, nullptr, perm, nullptr, 0, s);
+  launch_order_segments(cell_start, (int)ncells, nullptr, perm, nullptr, 0, nullptr, 0, s);
 }

@@ -313,6 +313,7 @@ static void swarm_replaced(FdfContext *ctx) {
   ctx->swarm_set = true;
   ctx->layout_ok = false;
   ctx->unsorted = 0;
+  ctx->maybe_nowhere = true;
 }
 
 // The swarm buffers from particle `off` on.
@@ -680,8 +681,9 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
     // far_cells away get a learned guess, and the reference walk from P1 (k_locate32_path)
     // fetches the rows of the path toward the guess ahead of its evaluations
     LocatorState &L = ctx->loc;
+    const bool from_nowhere = !advect || ctx->maybe_nowhere;   // the walks may cross the grid
     launch_locate32(src, ctx->cap, g, ctx->table32, ctx->planes, ctx->dt, advect, ctx->bbox, ctx->fbox, drop,
-                    ctx->cnt, ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, L.pflag, L.far_cells, s);
+                    ctx->cnt, ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, L.pflag, L.far_cells, from_nowhere, s);
     const long long nw = ((long long)ctx->cap + 31) / 32;   // the warps' pending counts, scanned in place
     ctx->launches += exclusive_scan_u32(L.pflag + nw, nw + 1, L.scan_sums, s) + 3;   // and these three
     launch_compact_pending(L.pflag, ctx->cap, L.pending, ctx->cnt, s);
@@ -690,10 +692,10 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
                  ctx->cap, g, L.guess, ctx->num_sms, &ctx->cnt->err, s);
     eg1 = prof ? record_event(ctx, s) : 0;
     launch_locate32_path(src, ctx->cap, g, ctx->table32, ctx->planes, ctx->bbox, ctx->fbox, drop, ctx->cnt,
-                         ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, L.pending, L.guess, ctx->num_sms, s);
+                         ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, L.pending, L.guess, ctx->num_sms, from_nowhere, s);
   } else if (f32) {
     launch_locate32(src, ctx->cap, g, ctx->table32, ctx->planes, ctx->dt, advect, ctx->bbox, ctx->fbox, drop,
-                    ctx->cnt, ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, nullptr, 0.f, s);
+                    ctx->cnt, ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, nullptr, 0.f, false, s);
   } else {
     launch_locate(src, ctx->cap, g, ctx->table32, ctx->planes, ctx->dt, advect, ctx->bbox, drop, ctx->cnt,
                     ctx->keys, ctx->rank, ctx->hist, ctx->sentinel, s);
@@ -774,7 +776,11 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
   ctx->layout_ok = true;
   ctx->unsorted = 0;
   ctx->launches += locate_only ? 2 : 4;   // slots, gather; corner field, deposit
-  return info ? read_info(ctx, info) : FDF_SUCCESS;
+  ctx->maybe_nowhere = !drop;             // a step drops the LOST
+  if (!info) return FDF_SUCCESS;
+  const int r = read_info(ctx, info);
+  if (!drop && r == FDF_SUCCESS) ctx->maybe_nowhere = ctx->cnt_host->lost_total > 0;
+  return r;
 }
 
 // Re-sorts the held particles by cell -- within a cell by PID in the plain form, in their
@@ -1085,6 +1091,7 @@ int fdf_AddParticles(FdfContext *ctx, int64_t n, const double *position, const d
   CU(cudaMemcpyAsync(&ctx->cnt->n_sorted, &total, sizeof(int), cudaMemcpyHostToDevice, s));
   CU(cudaStreamSynchronize(s));
   ctx->layout_ok = false;
+  ctx->maybe_nowhere = true;
   ctx->gen++;
   return FDF_SUCCESS;
 }
@@ -1136,9 +1143,10 @@ static int step_on_stream(FdfContext *ctx, int settled) {
   CU(cudaSetDevice(ctx->device));
   CU(cudaStreamIsCapturing(ctx->stream, &capturing));
   if (ctx->eager_gen != ctx->gen) ctx->eager_steps = 0;   // one-time set-up stays out of the capture
+  if (capturing != cudaStreamCaptureStatusNone) ctx->maybe_nowhere = false;   // what is recorded stands for later steps
   if (ctx->profiling || capturing != cudaStreamCaptureStatusNone ||
       (ctx->eager_steps < settled && ctx->graph_gen[ctx->cur] != ctx->gen) ||
-      (ctx->swarm_form == FDF_FORM_LEARNED_FP32 && !ctx->loc.has_params)) {
+      (ctx->swarm_form == FDF_FORM_LEARNED_FP32 && (!ctx->loc.has_params || ctx->maybe_nowhere))) {
     const int r = run_pipeline(ctx, 1, 1, nullptr);
     if (r) return r;
     ctx->eager_gen = ctx->gen;

@@ -71,6 +71,7 @@ struct FdfContext {
   unsigned int sentinel = 0;
   bool swarm_set = false;
   int64_t unsorted = 0;     // particles seeded (in no order of cells) and not yet sorted, else 0
+  bool maybe_nowhere = false;   // a held particle may have no cell (LOST kept by a setup, or set so by the caller)
   bool layout_ok = false;   // the held particles are sorted by cell and cell_start matches them
   int swarm_form = FDF_FORM_PLAIN_FP64;   // form the swarm's device arrays are held in
   int out_form = FDF_FORM_PLAIN_FP64;     // form of the last deposits

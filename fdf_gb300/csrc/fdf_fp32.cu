@@ -138,7 +138,8 @@ __device__ __forceinline__ unsigned int settle_key32(bool lost, int cell, float2
 }
 
 // Advect + locate, one thread per particle.
-//   FAR: the walks may start far from the particles (walk_ref32).
+//   FAR: the walks may start far from the particles (walk_ref32): without the advection and, in the learned form,
+//        where particles may have no previous cell.
 //   FIRST == false: the reference walk from the previous cell (or cell (0,0,0)).
 //   FIRST == true:  the reference's first evaluation, in the previous cell; a particle that it
 //                   does not conclude and that lies at least far_cells past that cell is
@@ -256,6 +257,11 @@ __device__ __forceinline__ void prefetch_row_l1(const float *row) {   // a row i
   asm volatile("prefetch.global.L1 [%0];" ::"l"(row));
 }
 
+// FAR: in a run that may hold particles without a previous cell (walk_ref32): one of them, whose walk crosses
+// the grid, holds the whole launch.  First step after a setup that kept 3,000 LOST of 100,000 (1024 cells along
+// k): 2.13 ms without, 1.08 with; elsewhere the registers of those evaluations cost more (64M particles, 527
+// against 534 us).
+template <bool FAR>
 __global__ void __launch_bounds__(FDF_GUESS_THREADS, FDF_GUESS_MIN_BLOCKS) k_locate32_path(SwarmBuf b, GridDims g, const float *__restrict__ table,
                                                         const double *__restrict__ planes,
                                                         const double *__restrict__ bbox,
@@ -288,7 +294,8 @@ __global__ void __launch_bounds__(FDF_GUESS_THREADS, FDF_GUESS_MIN_BLOCKS) k_loc
         if (ci == gi && cj == gj && ck == gk) break;   // the predicted path has reached the guess
       }
       Path32 path{w.i, w.j, w.k, gi, gj, gk, 0u};
-      walk_ref32<false, true>(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL - 1, w, cnt, 0.0, 0.0, 0.0, &path);
+      walk_ref32<false, true, false, FAR>(table, planes, g, px, py, pz, FDF_MAX_TRAVERSAL - 1, w, cnt, 0.0, 0.0, 0.0,
+                                          &path);
       hits += path.hits;
       if (w.degenerate) m.err |= ERRBIT_DEGENERATE;
       pev += w.evaluated();
@@ -788,7 +795,7 @@ void launch_build_table32(const double *planes, const double *coor, GridDims g, 
 void launch_locate32(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes, double dt,
                      int advect, const double *bbox, const float *fbox, int drop_removed, DevCounters *cnt,
                      unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
-                     unsigned int *pending, float far_cells, cudaStream_t s) {
+                     unsigned int *pending, float far_cells, bool from_nowhere, cudaStream_t s) {
   constexpr int th = FDF_LOC_THREADS;
   auto go = [&](auto kernel, unsigned int *pend, float far) {
     kernel<<<blocks_for(n_cap, th), th, 0, s>>>(b, g, table, planes, (float)dt, advect, drop_removed, bbox, fbox,
@@ -796,8 +803,8 @@ void launch_locate32(const SwarmBuf &b, int n_cap, GridDims g, const float *tabl
   };
   // without the advection the particles come from anywhere (the initial setup's corner start)
   const bool dense = n_cap > g.Nc;
-  if (pending && advect && dense) go(k_locate32<true, false, true>, pending, far_cells);
-  else if (pending && advect) go(k_locate32<true, false, false>, pending, far_cells);
+  if (pending && !from_nowhere && dense) go(k_locate32<true, false, true>, pending, far_cells);
+  else if (pending && !from_nowhere) go(k_locate32<true, false, false>, pending, far_cells);
   else if (pending) go(k_locate32<true, true, false>, pending, far_cells);
   else if (advect && dense) go(k_locate32<false, false, true>, nullptr, 0.f);
   else if (advect) go(k_locate32<false, false, false>, nullptr, 0.f);
@@ -812,19 +819,21 @@ void launch_compact_pending(const unsigned int *scan, int n_cap, unsigned int *l
 void launch_locate32_path(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes,
                           const double *bbox, const float *fbox, int drop_removed, DevCounters *cnt,
                           unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
-                          const unsigned int *pending, const int *guess, int num_sms, cudaStream_t s) {
+                          const unsigned int *pending, const int *guess, int num_sms, bool from_nowhere,
+                          cudaStream_t s) {
   // grid-stride kernel: one wave of resident blocks, so that no SM runs a partial last wave
   static int resident = 0, res_device = -1;
   int dev = 0;
   cudaGetDevice(&dev);
   if (res_device != dev) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_locate32_path, FDF_GUESS_THREADS, 0);
-    res_device = dev;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_locate32_path<false>, FDF_GUESS_THREADS, 0);
+    res_device = dev;   // (the same launch bounds: the same for <true>)
   }
   const long long need = ((long long)n_cap + FDF_GUESS_THREADS - 1) / FDF_GUESS_THREADS;
   long long blocks = (long long)num_sms * (resident > 0 ? resident : 1);
   if (blocks > need) blocks = need;
-  k_locate32_path<<<(unsigned)(blocks < 1 ? 1 : blocks), FDF_GUESS_THREADS, 0, s>>>(
+  auto *kernel = from_nowhere ? k_locate32_path<true> : k_locate32_path<false>;
+  kernel<<<(unsigned)(blocks < 1 ? 1 : blocks), FDF_GUESS_THREADS, 0, s>>>(
       b, g, table, planes, bbox, fbox, drop_removed, cnt, keys, rank, count, sentinel, pending, guess,
       FDF_PATH_LOOKAHEAD);
 }

@@ -271,7 +271,7 @@ void launch_build_table32(const double *planes, const double *coor, GridDims g, 
 void launch_locate32(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes, double dt,
                      int advect, const double *bbox, const float *fbox, int drop_removed, DevCounters *cnt,
                      unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
-                     unsigned int *pending, float far_cells, cudaStream_t s);
+                     unsigned int *pending, float far_cells, bool from_nowhere, cudaStream_t s);
 // The learned form's pending list from the warps' masks and scanned counts (sets cnt->pending).
 void launch_compact_pending(const unsigned int *scan, int n_cap, unsigned int *list, DevCounters *cnt,
                             cudaStream_t s);
@@ -280,7 +280,8 @@ void launch_compact_pending(const unsigned int *scan, int n_cap, unsigned int *l
 void launch_locate32_path(const SwarmBuf &b, int n_cap, GridDims g, const float *table, const double *planes,
                           const double *bbox, const float *fbox, int drop_removed, DevCounters *cnt,
                           unsigned int *keys, unsigned int *rank, unsigned int *count, unsigned int sentinel,
-                          const unsigned int *pending, const int *guess, int num_sms, cudaStream_t s);
+                          const unsigned int *pending, const int *guess, int num_sms, bool from_nowhere,
+                          cudaStream_t s);
 void launch_center_to_corner32(const float *ucat, GridDims g, float *corner, cudaStream_t s);
 void launch_gather_interp32(const SwarmBuf &src, const SwarmBuf &dst, int n_cap, GridDims g, const float *corner,
                             const unsigned int *perm, const unsigned int *cell_start, DevCounters *cnt,

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from fdf_gb300 import workloads as W
-from fdf_gb300.context import FORM_FP32, FORM_PLAIN_FP64, PicContext
+from fdf_gb300.context import FORM_FP32, FORM_LEARNED_FP32, FORM_PLAIN_FP64, PicContext
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +44,32 @@ def test_deposit_of_a_small_crowded_grid(require_gpu, dims, per_cell, momentum):
             ctx.initial_setup()
             t[form] = least(ctx.scatter, ctx.synchronize)
     assert t[FORM_PLAIN_FP64] < 3.4 * t[FORM_FP32], t
+
+
+def test_first_learned_step_after_a_setup_with_lost_particles(require_gpu):
+    """A LOST particle's walk from cell (0,0,0) holds the step.  With its open cells evaluated one walk behind another the
+    learned form's first step took 2.3 times the FP32 form's, in the loop 1.1."""
+    coor = W.sinusoidal_grid(64, 64, 1024)
+    ucat = W.field_taylor_green(W.cell_centroids(coor))
+    dt = W.min_edge_length(coor) / np.abs(ucat).max()
+    t = {}
+    for form in (FORM_FP32, FORM_LEARNED_FP32):
+        with PicContext(0) as ctx:
+            ctx.set_form(form)
+            ctx.set_grid(coor)
+            ctx.set_ucat(ucat)
+            ctx.set_dt(dt)
+            ctx.set_volume(1e-6)
+            if form == FORM_LEARNED_FP32:
+                ctx.locator_train(50_000, seed=1, steps=500, batch=4096)
+            out = []
+            for seed in range(4):
+                ctx.seed_particles(100_000, seed)
+                ctx.initial_setup()
+                ctx.synchronize()
+                t0 = time.perf_counter()
+                lost = ctx.step().removed_lost
+                out.append(time.perf_counter() - t0)
+                assert lost > 1000
+            t[form] = min(out[1:])
+    assert t[FORM_LEARNED_FP32] < 1.7 * t[FORM_FP32], t

@@ -1234,16 +1234,16 @@ int fdf_SortByCell(const int32_t *cell_ids, int64_t n, int64_t ncells, uint32_t 
   if (!cell_start) return FDF_ERR_ARG_NULL;
   if (n < 0 || n > FDF_MAX_PARTICLES || ncells < 1 || ncells + 1 > scan_max_count()) return FDF_ERR_ARG_OUTOFRANGE;
   cudaStream_t s = (cudaStream_t)stream;
-  // one allocation: the scan's sums, then the slots' ranks or, where there is no room for these, the
-  // cells' cursors
+  // one allocation: the scan's sums, then the cells' cursors (many ids per cell) or the slots' ranks and,
+  // where there is no room for these, cursors again
   const size_t nsums = (scan_scratch_words(ncells + 1) + 63) / 64 * 64;
   unsigned int *sums = nullptr;
-  bool ranks = true;
-  if (cudaMallocAsync((void **)&sums, 4ull * (nsums + n), s) != cudaSuccess) {
+  bool ranks = !cell_sort_by_tiles(n, ncells);
+  if (ranks && cudaMallocAsync((void **)&sums, 4ull * (nsums + n), s) != cudaSuccess) {
     (void)cudaGetLastError();
     ranks = false;
-    if (cudaMallocAsync((void **)&sums, 4ull * (nsums + ncells), s) != cudaSuccess) return FDF_ERR_MEM;
   }
+  if (!ranks && cudaMallocAsync((void **)&sums, 4ull * (nsums + ncells), s) != cudaSuccess) return FDF_ERR_MEM;
   cell_sort_on_scratch(cell_ids, n, ncells, perm, cell_start, ranks ? sums + nsums : nullptr,
                        ranks ? nullptr : sums + nsums, sums, s);
   cudaError_t e = cudaGetLastError();

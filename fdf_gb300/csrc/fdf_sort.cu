@@ -534,36 +534,42 @@ __global__ void __launch_bounds__(256) k_cell_rank(const int *__restrict__ cell,
   }
 }
 
-// The same for ids nearly in order (a step's ids are: a particle moves a few cells): a block whose
-// RANK_TILE ids span fewer than RANK_BINS cells counts them in shared memory, adds its counts to count[]
-// cell by cell -- neighbouring lanes on neighbouring words, one request where k_cell_rank makes 32 -- and
-// has its ids' ranks from the counts before them there and in the block.  A block whose ids span more
-// takes k_cell_rank's way.  Bound by the latency of its four phases: 32 registers (an id and its place share
-// a word) and four blocks an SM against two, 57 against 89 us for 16M ids in 4M cells, k_cell_rank 126 us.
+// A tile of TILE ids at a time, for ids nearly in order (a step's ids are: a particle moves a few cells): a block
+// whose ids span fewer than TILE_BINS cells counts them in shared memory and adds its counts to count[] cell
+// by cell -- neighbouring lanes on neighbouring words, one request where k_cell_rank makes 32.  SLOTS: the
+// second pass, which counts again, takes the block's place in each cell from `count` (the cells' cursors,
+// cell_start before) and writes the slots: nothing is kept per id between the passes, so the scratch is a
+// word per cell, a third of a word per id at most.  A block whose ids span more merges runs of equal
+// neighbours in a warp, as k_cell_rank does.  Bound by the latency of its phases: 32 registers and four
+// blocks an SM.
+// The whole sort with a rank kept per id between the passes, and now: 16M nearly sorted ids in 4M cells 191 -> 174
+// us (each call after a synchronisation, which gives the scratch back: 408 -> 333), 32M in 1M 663 -> 628 (1011 ->
+// 788), 64M in 14M 635 -> 542 (1217 -> 778); 16M in no order 393 -> 397 (608 -> 555), 32M in 1M 1339 -> 1196 (1681
+// -> 1360); 16M in runs of 8 and of 32 at random 298 -> 180 and 424 -> 218, one id in 8192 far off 249 -> 157.
 // From three ids per cell on, where a tile of ids in order spans 2731 cells and leaves the rest of the bins
-// for its disorder, and from 3M ids, half a wave of blocks.  The whole sort, before and with tiles: 16M ids
-// displaced by up to 4096 of 4M cells 394 -> 314 us, 32M of 2M cells 813 -> 652, 8M by up to 64 of 330k
-// 228 -> 194, 3.5M of 1M 149 -> 144; not used: 1M of 250k 224 -> 224 and, where blocks span too much, 16M
-// by up to 4096 of 14M cells 484 -> 515, 32M by up to 1M of 14M 826 -> 900 (16M of 4M 426 -> 433).
-constexpr int RANK_THREADS = 512, RANK_ITEMS = 16, RANK_TILE = RANK_THREADS * RANK_ITEMS, RANK_BINS = 12224;
-constexpr long long RANK_TILE_MIN = 3 << 20;
-__global__ void __launch_bounds__(RANK_THREADS, 4) k_cell_rank_tile(const int *__restrict__ cell, long long n,
-                                                                 long long ncells, unsigned int *__restrict__ count,
-                                                                 unsigned int *__restrict__ rank) {
-  __shared__ unsigned int bin[RANK_BINS];
+// for its disorder, and from 6M ids: against k_cell_rank and k_cell_place 102 for 118 us nearly sorted and 199 for
+// 187 in no order at 8M ids (3.1 per cell), 68 for 66 and 107 for 92 at 3.2M; at two per cell 111 for 125, 210 for
+// 202 at 8M, at one 161 for 158, 271 for 234.
+constexpr int TILE_THREADS = 512, TILE_ITEMS = 16, TILE = TILE_THREADS * TILE_ITEMS, TILE_BINS = 12224;
+constexpr long long TILE_MIN = 6 << 20;
+template <bool SLOTS>
+__global__ void __launch_bounds__(TILE_THREADS, 4) k_cell_tile(const int *__restrict__ cell, long long n, long long ncells,
+                                                             unsigned int *__restrict__ count,
+                                                             unsigned int *__restrict__ perm) {
+  __shared__ unsigned int bin[TILE_BINS];
   __shared__ unsigned int span[2];
-  const long long base = (long long)blockIdx.x * RANK_TILE + threadIdx.x;
+  const long long base = (long long)blockIdx.x * TILE + threadIdx.x;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) { span[0] = 0xffffffffu; span[1] = 0u; }
-  unsigned int key[RANK_ITEMS], lo = 0xffffffffu, hi = 0u;
+  unsigned int key[TILE_ITEMS], lo = 0xffffffffu, hi = 0u;
 #pragma unroll
-  for (int q = 0; q < RANK_ITEMS; ++q) {
-    const long long s = base + q * RANK_THREADS;
+  for (int q = 0; q < TILE_ITEMS; ++q) {
+    const long long s = base + q * TILE_THREADS;
     const int c = s < n ? cell[s] : -1;
     key[q] = c >= 0 && (long long)c < ncells ? (unsigned int)c : 0xffffffffu;
   }
 #pragma unroll
-  for (int q = 0; q < RANK_ITEMS; ++q) {
+  for (int q = 0; q < TILE_ITEMS; ++q) {
     lo = min(lo, key[q]);
     if (key[q] != 0xffffffffu) hi = max(hi, key[q]);
   }
@@ -576,35 +582,55 @@ __global__ void __launch_bounds__(RANK_THREADS, 4) k_cell_rank_tile(const int *_
   hi = span[1];
   if (lo == 0xffffffffu) return;   // no id of the block has a cell
   const unsigned int bins = hi - lo + 1u;
-  if (bins <= (unsigned int)RANK_BINS) {
-    for (unsigned int b = threadIdx.x; b < bins; b += RANK_THREADS) bin[b] = 0u;
+  if (bins <= (unsigned int)TILE_BINS) {
+    for (unsigned int b = threadIdx.x; b < bins; b += TILE_THREADS) bin[b] = 0u;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < RANK_ITEMS; ++q)   // from here on the bin and, above it, the id's place in it
+    for (int q = 0; q < TILE_ITEMS; ++q)   // SLOTS: from here on the bin and, above it, the id's place in it
       if (key[q] != 0xffffffffu) {
         key[q] -= lo;
-        key[q] |= atomicAdd(&bin[key[q]], 1u) << 16;
+        const unsigned int place = atomicAdd(&bin[key[q]], 1u);
+        if (SLOTS) key[q] |= place << 16;
       }
     __syncthreads();
 #pragma unroll 8
-    for (unsigned int b = threadIdx.x; b < bins; b += RANK_THREADS) {
+    for (unsigned int b = threadIdx.x; b < bins; b += TILE_THREADS) {
       const unsigned int c = bin[b];
-      if (c != 0u) bin[b] = atomicAdd(count + lo + b, c);
+      if (c != 0u) {
+        const unsigned int before = atomicAdd(count + lo + b, c);
+        if (SLOTS) bin[b] = before;
+      }
     }
+    if (!SLOTS) return;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < RANK_ITEMS; ++q)
-      if (key[q] != 0xffffffffu) rank[base + q * RANK_THREADS] = bin[key[q] & 0xffffu] + (key[q] >> 16);
+    for (int q = 0; q < TILE_ITEMS; ++q)
+      if (key[q] != 0xffffffffu) perm[bin[key[q] & 0xffffu] + (key[q] >> 16)] = (unsigned int)(base + q * TILE_THREADS);
     return;
   }
+  constexpr int IN_FLIGHT = 4;
 #pragma unroll
-  for (int h = 0; h < RANK_ITEMS; h += 4) {
-    unsigned int r[4];
+  for (int h = 0; h < TILE_ITEMS; h += IN_FLIGHT) {
+    unsigned int at[IN_FLIGHT];
+    int leader[IN_FLIGHT];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) r[q] = key[h + q] != 0xffffffffu ? atomicAdd(count + key[h + q], 1u) : 0u;
+    for (int q = 0; q < IN_FLIGHT; ++q) {
+      const unsigned int k = key[h + q], before = __shfl_up_sync(0xffffffffu, k, 1);
+      const unsigned int heads = __ballot_sync(0xffffffffu, lane == 0 || k != before);
+      const unsigned int upto = 0xffffffffu >> (31 - lane), later = heads & ~upto;
+      leader[q] = 31 - __clz((int)(heads & upto));
+      at[q] = 0u;
+      if (leader[q] == lane && k != 0xffffffffu)
+        at[q] = atomicAdd(count + k, (unsigned int)((later ? __ffs((int)later) - 1 : 32) - lane));
+    }
+    if (SLOTS) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (key[h + q] != 0xffffffffu) rank[base + (h + q) * RANK_THREADS] = r[q];
+      for (int q = 0; q < IN_FLIGHT; ++q) {
+        const unsigned int first = __shfl_sync(0xffffffffu, at[q], leader[q]);
+        if (key[h + q] != 0xffffffffu)
+          perm[first + (unsigned int)(lane - leader[q])] = (unsigned int)(base + (h + q) * TILE_THREADS);
+      }
+    }
   }
 }
 
@@ -629,9 +655,8 @@ __global__ void __launch_bounds__(256) k_cell_place(const int *__restrict__ cell
     if (c[q] >= 0) perm[at[q]] = (unsigned int)(base + (long long)q * blockDim.x);
 }
 
-// slot of every particle with a valid cell (warp-aggregated cursors)
+// slot of every particle with a valid cell (warp-aggregated cursors, the cells' starts before)
 __global__ void __launch_bounds__(256) k_cell_slots(const int *__restrict__ cell, long long n, long long ncells,
-                                                   const unsigned int *__restrict__ cell_start,
                                                    unsigned int *__restrict__ cursor, unsigned int *__restrict__ perm) {
   const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned int key = 0xffffffffu;
@@ -647,7 +672,7 @@ __global__ void __launch_bounds__(256) k_cell_slots(const int *__restrict__ cell
   unsigned int base = 0;
   if (lane == leader) base = atomicAdd(cursor + key, (unsigned int)__popc(peers));
   base = __shfl_sync(peers, base, leader);
-  perm[cell_start[key] + base + rank] = (unsigned int)s;
+  perm[base + rank] = (unsigned int)s;
 }
 
 }  // namespace
@@ -656,8 +681,10 @@ size_t scan_scratch_words(long long count) { return (size_t)((count + SCAN_BLOCK
 
 long long scan_max_count() { return (long long)SCAN_BLOCK * SCAN_THREADS * SUMS_PER_THREAD; }
 
-// Blocks of a scan whose offsets each block adds up itself: up to here (33M values) the launch saved
-// (2.5 us) outweighs the sums read again, half the blocks' count by each (14M cells: 3 MB in all).
+// Blocks of a scan whose offsets each block adds up itself, half of the sums on average: up to here (33M
+// values, 34 MB of sums read from L2 in all) the launch saved outweighs that.  A sort of 1000 ids, which is
+// its scan: 73 us against 75 with three launches in 8M cells, 100 against 103 in 14M, 153 against 158 in 24M,
+// 223 against 227 in 33M.
 constexpr long long SCAN_DIRECT = 4096;
 
 static int exclusive_scan(unsigned int *in, unsigned int *out, long long count, unsigned int *sums, int clear,
@@ -700,29 +727,27 @@ int launch_order_segments(const unsigned int *cell_start, int ncells, const long
   return 2;
 }
 
+bool cell_sort_by_tiles(long long n, long long ncells) { return n >= TILE_MIN && n >= 3 * ncells; }
+
 // Stable counting sort of particle slots by cell id, on caller-provided scratch: sums
-// [scan_scratch_words(ncells + 1)] and rank [n] or, where that is too much, cursor [ncells] (the
-// slots then come from a second pass of atomics).  cell_start [ncells + 1] is both the histogram and
-// (after the scan) the output.
+// [scan_scratch_words(ncells + 1)] and cursor [ncells] or, where cell_sort_by_tiles does not hold, rank [n]
+// (with a cursor the slots then come from a second pass of atomics).  cell_start [ncells + 1] is both the
+// histogram and (after the scan) the output.
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
                           unsigned int *cell_start, unsigned int *rank, unsigned int *cursor, unsigned int *sums,
                           cudaStream_t s) {
   const int th = 256;
   const unsigned int blocks = (unsigned int)std::max<long long>((n + th - 1) / th, 1);
-  const unsigned int blocks_items = (blocks + SORT_ITEMS - 1) / SORT_ITEMS;
+  const unsigned int blocks_items = (blocks + SORT_ITEMS - 1) / SORT_ITEMS, tiles = (unsigned int)((n + TILE - 1) / TILE);
+  const bool by_tiles = cursor && cell_sort_by_tiles(n, ncells);
   cudaMemsetAsync(cell_start, 0, 4ull * (ncells + 1), s);
-  if (rank) {
-    if (n >= RANK_TILE_MIN && n >= 3 * ncells)
-      k_cell_rank_tile<<<(unsigned int)((n + RANK_TILE - 1) / RANK_TILE), RANK_THREADS, 0, s>>>(cell, n, ncells,
-                                                                                                cell_start, rank);
-    else
-      k_cell_rank<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank);
-  } else {
-    cudaMemsetAsync(cursor, 0, 4ull * ncells, s);
-    k_cell_histogram<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start);
-  }
+  if (by_tiles) k_cell_tile<false><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cell_start, nullptr);
+  else if (rank) k_cell_rank<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank);
+  else k_cell_histogram<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start);
   exclusive_scan_u32(cell_start, ncells + 1, sums, s);
-  if (rank) k_cell_place<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank, perm);
-  else k_cell_slots<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start, cursor, perm);
+  if (cursor) cudaMemcpyAsync(cursor, cell_start, 4ull * ncells, cudaMemcpyDeviceToDevice, s);
+  if (by_tiles) k_cell_tile<true><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cursor, perm);
+  else if (rank) k_cell_place<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank, perm);
+  else k_cell_slots<<<blocks, th, 0, s>>>(cell, n, ncells, cursor, perm);
   launch_order_segments(cell_start, (int)ncells, nullptr, perm, nullptr, 0, nullptr, 0, s);
 }

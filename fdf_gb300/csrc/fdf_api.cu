@@ -63,8 +63,7 @@ int fdf_ContextCreate(FdfContext **out, int device) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_xfer, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->cnt, sizeof(DevCounters));
   if (e == cudaSuccess) e = cudaMemset(ctx->cnt, 0, sizeof(DevCounters));
-  if (e == cudaSuccess) e = cudaHostAlloc((void **)&ctx->cnt_host, DEVCOUNTERS_HEAD, cudaHostAllocDefault);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->bbox, 6 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->bbox, 7 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->fbox, 16 * sizeof(float));
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) {
@@ -87,7 +86,7 @@ int fdf_ContextDestroy(FdfContext *ctx) {
   if (ctx->side) cudaStreamSynchronize(ctx->side);
   cfree(ctx->swarm_mem); cfree(ctx->keys); cfree(ctx->perm); cfree(ctx->rank);
   cfree(ctx->hist); cfree(ctx->cell_start); cfree(ctx->scan_sums); cfree(ctx->cnt); cfree(ctx->staging);
-  if (ctx->cnt_host) cudaFreeHost(ctx->cnt_host);
+  if (ctx->cnt_locked) cudaFreeHost(ctx->cnt_locked);
   work_release(ctx);
   locator_free(ctx);
   for (auto &gx : ctx->step_graph)
@@ -160,8 +159,9 @@ int fdf_SetGrid(FdfContext *ctx, int64_t IM, int64_t JM, int64_t KM, const doubl
   CU(cudaMemsetAsync(ctx->ucat, 0, 24ull * Nc, ctx->stream));
   CU(cudaMemsetAsync(ctx->corner, 0, 24ull * Nn, ctx->stream));
   CU(cudaMemcpyAsync(ctx->coor, coor, 24ull * Nn, cudaMemcpyHostToDevice, ctx->stream));
-  unsigned int *err = nullptr;
-  launch_build_planes(ctx->coor, g, ctx->planes, err, ctx->stream);
+  ctx->degenerate = -1;
+  CU(cudaMemsetAsync(ctx->bbox + 6, 0, sizeof(double), ctx->stream));
+  launch_build_planes(ctx->coor, g, ctx->planes, (unsigned int *)(ctx->bbox + 6), ctx->stream);
   CHECK_LAUNCH();
   launch_build_table32(ctx->planes, ctx->coor, g, ctx->table32, ctx->stream);
   CHECK_LAUNCH();
@@ -498,9 +498,10 @@ int fdf_SeedParticles(FdfContext *ctx, int64_t n, uint64_t seed, int start_in_ge
 int fdf_GetSwarmSize(FdfContext *ctx, int64_t *n) {
   if (!ctx || !n) return fail(ctx, FDF_ERR_ARG_NULL, "fdf_GetSwarmSize: null argument");
   CU(cudaSetDevice(ctx->device));
-  CU(cudaMemcpyAsync(&ctx->cnt_host->n_sorted, &ctx->cnt->n_sorted, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  DevCounters *c = counts_host(ctx);
+  CU(cudaMemcpyAsync(&c->n_sorted, &ctx->cnt->n_sorted, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  *n = ctx->cnt_host->n_sorted;
+  *n = c->n_sorted;
   return FDF_SUCCESS;
 }
 
@@ -632,15 +633,16 @@ namespace {
 
 // The counts of the last pipeline run; waits for it.
 int read_info(FdfContext *ctx, FdfStepInfo *info) {
-  CU(cudaMemcpyAsync(ctx->cnt_host, ctx->cnt, DEVCOUNTERS_HEAD, cudaMemcpyDeviceToHost, ctx->stream));
+  const DevCounters &c = *counts_host(ctx);
+  CU(cudaMemcpyAsync((void *)&c, ctx->cnt, DEVCOUNTERS_HEAD, cudaMemcpyDeviceToHost, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
-  const DevCounters &c = *ctx->cnt_host;
   info->n_start = c.n_start;
   info->n_end = c.n_sorted;
   info->removed_lost = (int64_t)c.removed_lost;
   info->removed_oob = (int64_t)c.removed_oob;
   info->walk_evals = (int64_t)c.evals;
   info->fp64_fallbacks = (int64_t)c.fallbacks;
+  ctx->maybe_nowhere = ctx->maybe_nowhere && c.lost_total > 0;   // (of a setup or a staged call)
   if (c.err & ERRBIT_DEGENERATE)
     return fail(ctx, FDF_ERR_USER, "Degenerate plane detected (normal vector is near zero).");
   if (c.err & ERRBIT_TC_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "learned locator: tensor-core wait timed out");
@@ -778,9 +780,7 @@ int run_pipeline(FdfContext *ctx, int advect, int drop, FdfStepInfo *info, bool 
   ctx->launches += locate_only ? 2 : 4;   // slots, gather; corner field, deposit
   ctx->maybe_nowhere = !drop;             // a step drops the LOST
   if (!info) return FDF_SUCCESS;
-  const int r = read_info(ctx, info);
-  if (!drop && r == FDF_SUCCESS) ctx->maybe_nowhere = ctx->cnt_host->lost_total > 0;
-  return r;
+  return read_info(ctx, info);
 }
 
 // Re-sorts the held particles by cell -- within a cell by PID in the plain form, in their
@@ -931,19 +931,27 @@ int fdf_LocatePoints(FdfContext *ctx, int64_t n, const double *position, const i
   long long *d_cell = (long long *)(d_pos + 3ull * m);
   double *d_w = (double *)(d_cell + 3ull * m);
   long long *d_st = (long long *)(d_w + 3ull * m);
-  cudaError_t e = cudaMemcpyAsync(d_pos, position, aos, cudaMemcpyHostToDevice, s);
+  cudaError_t e = cudaSuccess;
+  if (ctx->degenerate < 0) {
+    unsigned int any = 0;
+    e = cudaMemcpyAsync(&any, ctx->bbox + 6, sizeof(any), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) ctx->degenerate = any ? 1 : 0;
+  }
+  const bool watch = ctx->degenerate != 0;   // else no walk can meet a degenerate cell
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_pos, position, aos, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && cell_in) e = cudaMemcpyAsync(d_cell, cell_in, aos, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(&tc->err, 0, sizeof(tc->err), s);
+  if (e == cudaSuccess && watch) e = cudaMemsetAsync(&tc->err, 0, sizeof(tc->err), s);
   if (e == cudaSuccess) {
     launch_locate_points(d_pos, cell_in ? d_cell : nullptr, m, g, ctx->table32, ctx->planes, tc, d_cell, d_w, d_st, s);
     ctx->launches += 1;
     e = cudaGetLastError();
   }
-  unsigned int &err = ctx->cnt_host->err;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&err, &tc->err, sizeof(err), cudaMemcpyDeviceToHost, s);
+  unsigned int err = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(cell_out, d_cell, aos, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(weight, d_w, aos, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(status, d_st, one, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess && watch) e = cudaMemcpyAsync(&err, &tc->err, sizeof(err), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(ctx, FDF_ERR_GPU, std::string("fdf_LocatePoints: ") + cudaGetErrorString(e));
   if (err & ERRBIT_DEGENERATE) return fail(ctx, FDF_ERR_USER, "Degenerate plane detected (normal vector is near zero).");

@@ -46,7 +46,7 @@ __device__ __forceinline__ bool face_plane(V3 v1, V3 v2, V3 v3, V3 v4, V3 cc, do
 }
 
 __global__ void k_build_planes(const double *__restrict__ coor, GridDims g, double *__restrict__ planes,
-                               unsigned int *err) {
+                               unsigned int *any_degenerate) {
   long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (c >= g.Nc) return;
   int i, j, k;
@@ -85,7 +85,7 @@ __global__ void k_build_planes(const double *__restrict__ coor, GridDims g, doub
   degen |= face_plane(v[1], v[2], v[5], v[6], cc, row + 6 * F_RIGHT);
   row[36] = thr;
   row[37] = degen ? 1.0 : 0.0;
-  (void)err;
+  if (degen) *any_degenerate = 1u;
 }
 
 // The corner field (fdf_corner.cuh), one thread per node.  With cell_start non-null, nodes none of
@@ -194,10 +194,10 @@ void launch_vec3_out(const float *soa, long long n, double *aos, cudaStream_t s)
   k_vec3_out<<<blocks_for(n), 256, 0, s>>>(soa, n, aos);
 }
 
-void launch_build_planes(const double *coor, GridDims g, double *planes, unsigned int *err, cudaStream_t s) {
+void launch_build_planes(const double *coor, GridDims g, double *planes, unsigned int *any_degenerate, cudaStream_t s) {
   int th = 128;
   long long blocks = (g.Nc + th - 1) / th;
-  k_build_planes<<<(unsigned)blocks, th, 0, s>>>(coor, g, planes, err);
+  k_build_planes<<<(unsigned)blocks, th, 0, s>>>(coor, g, planes, any_degenerate);
 }
 
 void launch_center_to_corner(const double *ucat, GridDims g, double *corner, const unsigned int *cell_start,

@@ -174,7 +174,8 @@ void launch_move_kept(const SwarmBuf &src, const SwarmBuf &dst, int a, int b, in
 // The plain form's k-faces of layer k summed again from seeds (fdf_DepositKFaceLayer).
 void launch_deposit_k_layer(const SwarmBuf &b, GridDims g, const unsigned int *cell_start, int k, double volume,
                             const double *seed, const double *seed_mom, double *fk, double *mk, cudaStream_t s);
-void launch_build_planes(const double *coor_aos, GridDims g, double *planes, unsigned int *err, cudaStream_t s);
+// any_degenerate is set to 1 where a cell has a degenerate face (zero before).
+void launch_build_planes(const double *coor_aos, GridDims g, double *planes, unsigned int *any_degenerate, cudaStream_t s);
 // cell_start == nullptr: every node; else only nodes adjacent to an occupied cell.
 void launch_center_to_corner(const double *ucat, GridDims g, double *corner, const unsigned int *cell_start,
                              unsigned long long *nodes_done, cudaStream_t s);

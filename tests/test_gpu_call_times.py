@@ -73,3 +73,44 @@ def test_first_learned_step_after_a_setup_with_lost_particles(require_gpu):
                 assert lost > 1000
             t[form] = min(out[1:])
     assert t[FORM_LEARNED_FP32] < 1.7 * t[FORM_FP32], t
+
+
+def test_a_context_costs_less_than_a_page_locked_block(require_gpu):
+    """Creating and closing a context: 130 us, 460 with a page-locked block in it (330 by itself), which only a run of many
+    steps earns back."""
+    import ctypes
+    drv = ctypes.CDLL("libcuda.so.1")
+    PicContext(0).close()   # the device's own context
+
+    def block():
+        p = ctypes.c_void_p()
+        assert drv.cuMemAllocHost_v2(ctypes.byref(p), 256) == 0
+        assert drv.cuMemFreeHost(p) == 0
+
+    def context():
+        PicContext(0).close()
+
+    nothing = lambda: None
+    for _ in range(5):
+        block()
+    t_block, t_context = (np.median([least(f, nothing, repeat=1) for _ in range(21)]) for f in (block, context))
+    assert t_context < t_block, (t_context, t_block)
+
+
+def test_counts_through_the_change_of_their_block(require_gpu):
+    """Steps' counts before, at and after the read from which they go to page-locked memory."""
+    wl = W.config_sinusoidal(IM=6, JM=6, KM=12, n=500, cfl=0.1, steps=1)
+    with PicContext(0) as a, PicContext(0) as b:
+        for ctx in (a, b):
+            ctx.load_workload(wl)
+        first = a.initial_setup()
+        b.initial_setup()
+        held = first.n_end
+        for q in range(140):
+            info = a.step()
+            b.step(info=False)
+            assert info.n_start == held
+            held = info.n_end
+            assert a.size() == held
+        assert b.size() == held
+        assert np.array_equal(a.get_swarm().pid, b.get_swarm().pid)

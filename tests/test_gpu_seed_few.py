@@ -1,0 +1,48 @@
+"""GPU: seeding on both sides of the count from which its products and conversions run on the integer pipe, bit for bit
+the host's generator; and its time for a hundred particles against a read of four bytes."""
+import time
+
+import numpy as np
+import pytest
+
+from fdf_gb300 import workloads as W
+from fdf_gb300.context import FORM_FP32, FORM_PLAIN_FP64, PicContext
+
+pytestmark = pytest.mark.gpu
+
+LINE = 3 << 14
+
+
+@pytest.mark.parametrize("form", [FORM_PLAIN_FP64, FORM_FP32])
+@pytest.mark.parametrize("n", [1, 33, LINE - 1, LINE, LINE + 1])
+def test_both_sides_are_the_host_generator(require_gpu, form, n):
+    coor = W.bent_pipe_grid(17, 9, 31)
+    pos, cell = W.volumetric_particles(coor, n, seed=11)
+    with PicContext(0) as ctx:
+        ctx.set_form(form)
+        ctx.set_grid(coor)
+        ctx.seed_particles(n, 11)
+        s = ctx.get_swarm()
+    if form == FORM_FP32:   # held as float pairs
+        hi = pos.astype(np.float32).astype(np.float64)
+        pos = hi + (pos - hi).astype(np.float32).astype(np.float64)
+    assert np.array_equal(s.position.view(np.int64), pos.view(np.int64))
+    assert np.array_equal(s.cell, cell)
+
+
+def test_a_hundred_particles(require_gpu):
+    """2.5 times the read on the integer pipe, 1.95 on the FP64 pipe."""
+    with PicContext(0) as ctx:
+        ctx.set_grid(W.uniform_grid(20, 20, 20))
+
+        def least(f):
+            out = []
+            for _ in range(400):
+                t0 = time.perf_counter()
+                f()
+                out.append(time.perf_counter() - t0)
+            return float(np.percentile(out[150:], 20))
+
+        ctx.seed_particles(100, 1)
+        read, seed = least(ctx.size), least(lambda: ctx.seed_particles(100, 1))
+    assert seed < 2.3 * read, (seed, read)

@@ -25,10 +25,20 @@ namespace {
 
 // Allocations left before dev_alloc starts failing (fdf_TestFailDeviceAllocations); -1: no limit.
 std::atomic<long long> g_alloc_budget{-1};
+// Allocations left before the one that fails (fdf_TestFailOneDeviceAllocation); -1: none.
+std::atomic<long long> g_alloc_one{-1};
 
 }  // namespace
 
+bool dev_alloc_one_fails() {
+  return g_alloc_one.load() >= 0 && g_alloc_one.fetch_sub(1) == 0;
+}
+
 cudaError_t dev_alloc_hooked(void **p, size_t bytes) {
+  if (dev_alloc_one_fails()) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
+  }
   long long b = g_alloc_budget.load();
   while (b >= 0) {
     if (b == 0) {
@@ -44,6 +54,11 @@ extern "C" {
 
 int fdf_TestFailDeviceAllocations(int64_t after) {
   g_alloc_budget.store(after < 0 ? -1 : (long long)after);
+  return FDF_SUCCESS;
+}
+
+int fdf_TestFailOneDeviceAllocation(int64_t after) {
+  g_alloc_one.store(after < 0 ? -1 : (long long)after);
   return FDF_SUCCESS;
 }
 
@@ -1121,7 +1136,7 @@ int fdf_DepositKFaceLayer(FdfContext *ctx, int64_t k, const double *seed, const 
   const long long L = (long long)g.IM * g.JM;
   const bool mom = ctx->out_momentum && ctx->mom;
   double *d = nullptr;
-  CU(cudaMalloc((void **)&d, 8ull * L * 4));
+  CU(ctx_alloc(ctx, &d, 8ull * L * 4));
   cudaStream_t s = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(d, seed, 8ull * L, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
@@ -1251,7 +1266,7 @@ int fdf_SortByCell(const int32_t *cell_ids, int64_t n, int64_t ncells, uint32_t 
   const size_t nsums = (scan_scratch_words(ncells + 1) + 63) / 64 * 64;
   unsigned int *sums = nullptr;
   bool ranks = !cell_sort_by_tiles(n, ncells);
-  if (ranks && cudaMallocAsync((void **)&sums, 4ull * (nsums + n), s) != cudaSuccess) {
+  if (ranks && (dev_alloc_one_fails() || cudaMallocAsync((void **)&sums, 4ull * (nsums + n), s) != cudaSuccess)) {
     (void)cudaGetLastError();
     ranks = false;
   }
@@ -1285,8 +1300,8 @@ int fdf_SetMomentumDeposit(FdfContext *ctx, int enable) {
     ctx->momentum = false;
     ctx->gen++;
     cfree(ctx->mom); cfree(ctx->mom32);
-    CU(dev_alloc(&ctx->mom, 24ull * nf));
-    CU(dev_alloc(&ctx->mom32, 12ull * nf));
+    CU(ctx_alloc(ctx, &ctx->mom, 24ull * nf));
+    CU(ctx_alloc(ctx, &ctx->mom32, 12ull * nf));
     CU(cudaMemset(ctx->mom, 0, 24ull * nf));
     CU(cudaMemset(ctx->mom32, 0, 12ull * nf));
   }

@@ -72,6 +72,7 @@ struct FdfContext {
   size_t staging_bytes = 0;
   void *work = nullptr;                   // CallBuffer's memory between calls
   size_t work_bytes = 0;
+  bool work_busy = false;                 // a call is using it
   int xfer_route = FDF_TRANSFER_AUTO;     // fdf_SetTransferRoute
   int route_up = -1, route_down = -1;     // AUTO: the route measured faster per direction (-1: not yet)
   unsigned int sentinel = 0;
@@ -161,38 +162,61 @@ inline void cfree(T *&p) {
 // can make them fail on the host (fdf_TestFailDeviceAllocations) and check that the context
 // is left refusing work instead of holding freed pointers.
 cudaError_t dev_alloc_hooked(void **p, size_t bytes);
+bool dev_alloc_one_fails();   // this is the one allocation that fdf_TestFailOneDeviceAllocation lets fail
 template <typename T>
 inline cudaError_t dev_alloc(T **p, size_t bytes) {
   return dev_alloc_hooked(reinterpret_cast<void **>(p), bytes);
 }
 
 
-// Device memory for the length of one call (points, predictions).  Up to WORK_MAX it stays with the
-// context for the next call (an allocation and its release cost 150 us), until fdf_SetGrid or
-// fdf_ReserveParticles need the room; a larger one is released at the call's end.
+inline void work_release(FdfContext *ctx) {
+  cfree(ctx->work);
+  ctx->work_bytes = 0;
+}
+
+// Device memory for a context: where there is no room, CallBuffer's kept memory goes first, unless the call
+// itself uses it.
+template <typename T>
+inline cudaError_t ctx_alloc(FdfContext *ctx, T **p, size_t bytes) {
+  cudaError_t e = dev_alloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && ctx->work && !ctx->work_busy) {
+    (void)cudaGetLastError();
+    work_release(ctx);
+    e = dev_alloc(p, bytes);
+  }
+  return e;
+}
+
+// Device memory for the length of one call (points, predictions, training's samples).  Up to WORK_MAX it
+// stays with the context for the next call (an allocation and its release cost 150 us), until fdf_SetGrid,
+// fdf_ReserveParticles or another allocation of the context need the room; a larger one is released at
+// the call's end.
 struct CallBuffer {
   static constexpr size_t WORK_MAX = size_t(256) << 20;
-  char *p = nullptr;
-  bool own = false;
+  FdfContext *user = nullptr;   // whose kept memory this is
+  char *p = nullptr;            // else its own
   cudaError_t take(FdfContext *ctx, size_t bytes) {
-    if (bytes <= ctx->work_bytes) {
-      p = (char *)ctx->work;
-      return cudaSuccess;
+    if (bytes > WORK_MAX) return ctx_alloc(ctx, &p, bytes);
+    if (bytes > ctx->work_bytes) {
+      work_release(ctx);
+      const cudaError_t e = dev_alloc(&ctx->work, bytes);
+      if (e != cudaSuccess) {
+        ctx->work = nullptr;
+        return e;
+      }
+      ctx->work_bytes = bytes;
     }
-    own = bytes > WORK_MAX;
-    if (own) return cudaMalloc((void **)&p, bytes);
-    cfree(ctx->work);
-    ctx->work_bytes = 0;
-    const cudaError_t e = cudaMalloc(&ctx->work, bytes);
-    if (e != cudaSuccess) return e;
-    ctx->work_bytes = bytes;
+    user = ctx;
+    user->work_busy = true;
     p = (char *)ctx->work;
     return cudaSuccess;
   }
   ~CallBuffer() {
-    if (own) cudaFree(p);
+    if (user) user->work_busy = false;
+    else if (p) cudaFree(p);
   }
 };
+
 // Where the counters' head is read to.
 inline DevCounters *counts_host(FdfContext *ctx) {
   if (ctx->cnt_reads < FdfContext::COUNTS_LOCKED && ++ctx->cnt_reads == FdfContext::COUNTS_LOCKED) {
@@ -205,11 +229,6 @@ inline DevCounters *counts_host(FdfContext *ctx) {
     cudaThreadExchangeStreamCaptureMode(&mode);
   }
   return ctx->cnt_locked ? ctx->cnt_locked : reinterpret_cast<DevCounters *>(ctx->cnt_page);
-}
-
-inline void work_release(FdfContext *ctx) {
-  cfree(ctx->work);
-  ctx->work_bytes = 0;
 }
 
 // Bytes of one swarm buffer, a multiple of 256: the second buffer of the pair starts at this

@@ -279,10 +279,10 @@ int device_metrics(FdfContext *ctx, double **metrics, double **aj, int *flipped)
   unsigned *err = nullptr;
   constexpr int MM_BLOCKS = 1024;
   auto cleanup = [&]() { cfree(m); cfree(a); cfree(part); cfree(err); };
-  cudaError_t e = cudaMalloc((void **)&m, 72ull * Nn);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&a, 8ull * Nn);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&part, 16ull * MM_BLOCKS);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&err, sizeof(unsigned));
+  cudaError_t e = ctx_alloc(ctx, &m, 72ull * Nn);
+  if (e == cudaSuccess) e = ctx_alloc(ctx, &a, 8ull * Nn);
+  if (e == cudaSuccess) e = ctx_alloc(ctx, &part, 16ull * MM_BLOCKS);
+  if (e == cudaSuccess) e = ctx_alloc(ctx, &err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemsetAsync(m, 0, 72ull * Nn, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(a, 0, 8ull * Nn, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream);
@@ -347,8 +347,8 @@ int ensure_c2c_table(FdfContext *ctx) {
   int r = device_metrics(ctx, &m, &a, &flipped);
   if (r) return r;
   unsigned *err = nullptr;
-  cudaError_t e = cudaMalloc((void **)&ctx->c2c_table, 8ull * C2C_SLOTS * g.Nc);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&err, sizeof(unsigned));
+  cudaError_t e = ctx_alloc(ctx, &ctx->c2c_table, 8ull * C2C_SLOTS * g.Nc);
+  if (e == cudaSuccess) e = ctx_alloc(ctx, &err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream);
   if (e == cudaSuccess) {
     k_c2c_table<<<blocks_of(g.Nc, 256), 256, 0, ctx->stream>>>(m, m + 3 * g.Nn, m + 6 * g.Nn, g, ctx->c2c_table, err);
@@ -413,7 +413,7 @@ int fdf_SetUcont(FdfContext *ctx, const double *ucont) {
   if (!ctx || !ucont) return fail(ctx, FDF_ERR_ARG_NULL, "fdf_SetUcont: null argument");
   if (!ctx->has_grid) return fail(ctx, FDF_ERR_ARG_WRONGSTATE, "fdf_SetUcont: call fdf_SetGrid first");
   CU(cudaSetDevice(ctx->device));
-  if (!ctx->ucont) CU(cudaMalloc((void **)&ctx->ucont, 24ull * ctx->g.Nn));
+  if (!ctx->ucont) CU(ctx_alloc(ctx, &ctx->ucont, 24ull * ctx->g.Nn));
   CU(cudaMemcpyAsync(ctx->ucont, ucont, 24ull * ctx->g.Nn, cudaMemcpyHostToDevice, ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
   return FDF_SUCCESS;

@@ -58,13 +58,13 @@ int alloc_params(FdfContext *ctx) {
   L.has_params = false;
   cfree(L.params); cfree(L.grads); cfree(L.adam_m); cfree(L.adam_v); cfree(L.train_img);
   cfree(L.bias); cfree(L.tc_img);
-  CU(dev_alloc(&L.params, 4ull * MLP_NPARAM));
-  CU(dev_alloc(&L.grads, 4ull * MLP_NPARAM));
-  CU(dev_alloc(&L.adam_m, 4ull * MLP_NPARAM));
-  CU(dev_alloc(&L.adam_v, 4ull * MLP_NPARAM));
-  CU(dev_alloc(&L.train_img, MLP_IMG_BYTES));
-  CU(dev_alloc(&L.bias, 4ull * MLP_BIAS_WORDS));
-  CU(dev_alloc(&L.tc_img, mlp_tc_image_bytes()));
+  CU(ctx_alloc(ctx, &L.params, 4ull * MLP_NPARAM));
+  CU(ctx_alloc(ctx, &L.grads, 4ull * MLP_NPARAM));
+  CU(ctx_alloc(ctx, &L.adam_m, 4ull * MLP_NPARAM));
+  CU(ctx_alloc(ctx, &L.adam_v, 4ull * MLP_NPARAM));
+  CU(ctx_alloc(ctx, &L.train_img, MLP_IMG_BYTES));
+  CU(ctx_alloc(ctx, &L.bias, 4ull * MLP_BIAS_WORDS));
+  CU(ctx_alloc(ctx, &L.tc_img, mlp_tc_image_bytes()));
   return FDF_SUCCESS;
 }
 
@@ -73,7 +73,7 @@ int ensure_scratch(FdfContext *ctx, int B) {
   if (L.batch_cap >= B && L.scratch) return FDF_SUCCESS;
   cfree(L.scratch);
   L.batch_cap = 0;
-  CU(dev_alloc(&L.scratch, scratch_bytes(B)));
+  CU(ctx_alloc(ctx, &L.scratch, scratch_bytes(B)));
   L.batch_cap = B;
   return FDF_SUCCESS;
 }
@@ -119,10 +119,10 @@ int locator_reserve(FdfContext *ctx) {
   if (L.pending_cap >= ctx->cap && L.pending) return FDF_SUCCESS;
   cfree(L.pending); cfree(L.guess); cfree(L.pflag); cfree(L.scan_sums);
   L.pending_cap = 0;
-  CU(dev_alloc(&L.pending, 4ull * ctx->cap));
-  CU(dev_alloc(&L.guess, 4ull * ctx->cap));
-  CU(dev_alloc(&L.pflag, 4ull * (2 * ((ctx->cap + 31) / 32) + 1)));
-  CU(dev_alloc(&L.scan_sums, 4ull * scan_scratch_words(ctx->cap + 1)));
+  CU(ctx_alloc(ctx, &L.pending, 4ull * ctx->cap));
+  CU(ctx_alloc(ctx, &L.guess, 4ull * ctx->cap));
+  CU(ctx_alloc(ctx, &L.pflag, 4ull * (2 * ((ctx->cap + 31) / 32) + 1)));
+  CU(ctx_alloc(ctx, &L.scan_sums, 4ull * scan_scratch_words(ctx->cap + 1)));
   L.pending_cap = ctx->cap;
   return FDF_SUCCESS;
 }

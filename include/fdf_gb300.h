@@ -218,7 +218,11 @@ int fdf_ScatterAllParticleFieldsToEulerFields(FdfContext *ctx);
  * that are not the swarm (probes, post-processing): the plain FP64 walk, bit-identical to the
  * reference, from cell_in[p] (or cell (0,0,0), a new particle's start, where it is -1 or
  * cell_in is NULL).  Outputs: cell_out [n][3] (-1 when LOST), weight [n][3] (zero when LOST),
- * status [n] (ACTIVE_AND_LOCATED or LOST).  Host arrays; the swarm is not touched. */
+ * status [n] (ACTIVE_AND_LOCATED or LOST).  Host arrays; the swarm is not touched.
+ * This call, fdf_InterpolatePoints, fdf_LocatorPredict and fdf_LocatorTrain share a device buffer that the
+ * context keeps for the next of them while it is no larger than 256 MB (fdf_LocatePoints: 80 bytes
+ * a point); fdf_SetGrid, a growing fdf_ReserveParticles, an allocation of the context that finds no
+ * room and fdf_ContextDestroy release it. */
 int fdf_LocatePoints(FdfContext *ctx, int64_t n, const double *position, const int64_t *cell_in, int64_t *cell_out,
                      double *weight, int64_t *status);
 
@@ -376,6 +380,9 @@ int fdf_GetStageTimes(FdfContext *ctx, double *ms_total, int64_t *launches, int 
  * grid (or no swarm) and returns FDF_ERR_ARG_WRONGSTATE from the calls that need one.
  * Process-wide; not for production use. */
 int fdf_TestFailDeviceAllocations(int64_t after);
+/* The same for one allocation, those of fdf_SortByCell among them: `after` succeed, the next
+ * one fails, later ones succeed again (a negative value: none fails). */
+int fdf_TestFailOneDeviceAllocation(int64_t after);
 /* Time-out path of the learned locator's tensor-core kernel: fdf_LocatorPredict's launch on n
  * positions [n][3] with no MMA issued, so that each CTA's first bounded mbarrier wait (1024
  * polls) runs out; the CTAs free their tensor memory and return, and the call returns

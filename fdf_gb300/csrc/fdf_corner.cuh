@@ -10,9 +10,8 @@
 
 namespace fdfx {
 
-// XI, YI, ZI: bit e puts the addition of the e-th cell to that component on the integer pipe (the same
-// bits).
-template <int XI, int YI, int ZI>
+// INT: bit e puts the addition of the e-th cell to each component on the integer pipe (the same bits).
+template <int INT>
 __device__ __forceinline__ void corner_value(const double *__restrict__ ucat, const GridDims &g, int i, int j, int k,
                                              double &ox, double &oy, double &oz) {
   const unsigned int IM = g.IM, JM = g.JM;
@@ -32,9 +31,9 @@ __device__ __forceinline__ void corner_value(const double *__restrict__ ucat, co
       if (e == 0) {
         sx = add0(vx); sy = add0(vy); sz = add0(vz);
       } else {
-        sx = (XI >> e & 1) ? add_int(sx, vx) : add(sx, vx);
-        sy = (YI >> e & 1) ? add_int(sy, vy) : add(sy, vy);
-        sz = (ZI >> e & 1) ? add_int(sz, vz) : add(sz, vz);
+        sx = (INT >> e & 1) ? add_int(sx, vx) : add(sx, vx);
+        sy = (INT >> e & 1) ? add_int(sy, vy) : add(sy, vy);
+        sz = (INT >> e & 1) ? add_int(sz, vz) : add(sz, vz);
       }
     }
   }

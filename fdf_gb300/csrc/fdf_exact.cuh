@@ -319,8 +319,7 @@ __device__ __forceinline__ double one_minus(double a) {
     A = 0ull;
     rest = 1u;
   }
-  const unsigned long long R = 0ull - A - rest;                     // 2^64 - a, truncated
-  if (R == 0ull) return 1.0;   // not reached: A = 0 comes with rest
+  const unsigned long long R = 0ull - A - rest;                     // 2^64 - a, truncated; not 0: A = 0 comes with rest
   const int lz = __clzll((long long)R);
   const unsigned long long n = R << lz, mant = n >> 11;
   const unsigned int low = ((unsigned int)n & 0x7ffu) * 2u + rest;   // the remainder in half units, sticky

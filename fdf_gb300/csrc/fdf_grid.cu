@@ -91,7 +91,7 @@ __global__ void k_build_planes(const double *__restrict__ coor, GridDims g, doub
 // The corner field (fdf_corner.cuh), one thread per node.  With cell_start non-null, nodes none of
 // whose adjacent cells holds a particle are skipped: the corner field is an intermediate of the
 // interpolation and only those nodes are ever read.
-// Bound by FP64 adds, 21 a node: of each component's seven two go to the integer pipe (masks 0x88: the
+// Bound by FP64 adds, 21 a node: of each component's seven two go to the integer pipe (mask 0x88: the
 // fourth and the eighth cell's), which then takes as long.  Per step 178 -> 132 us for 4.2M cells with 1M
 // particles, 628 -> 465 us for 14M with 16M (one component zero); with four to ten of the 21 there
 // 138/491, 137/448, 147/459, 157/489 us.  The lanes of a row's ends take the same path as the others, the
@@ -123,7 +123,7 @@ __global__ void k_center_to_corner(const double *__restrict__ ucat, GridDims g, 
   }
   if (!work) return;
   double ox, oy, oz;
-  fdfx::corner_value<0x88, 0x88, 0x88>(ucat, g, i, j, k, ox, oy, oz);
+  fdfx::corner_value<0x88>(ucat, g, i, j, k, ox, oy, oz);
   if (AOS) {
     corner[3 * q] = ox; corner[3 * q + 1] = oy; corner[3 * q + 2] = oz;
   } else {

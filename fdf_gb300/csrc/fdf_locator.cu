@@ -275,12 +275,12 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
                *flag = (unsigned int *)(buf.p + o_flag), *slot = (unsigned int *)(buf.p + o_slot),
                *sums = (unsigned int *)(buf.p + o_sums);
   float *xs = (float *)(buf.p + o_xs), *ts = (float *)(buf.p + o_ts), *hist_loss = (float *)(buf.p + o_loss);
-  auto release = [&]() { cudaStreamSynchronize(s); };
+  auto settle = [&]() { cudaStreamSynchronize(s); };   // what reads the buffer has ended
 #define CUT(call)                                                                    \
   do {                                                                               \
     cudaError_t e_ = (call);                                                         \
     if (e_ != cudaSuccess) {                                                         \
-      release();                                                                     \
+      settle();                                                                     \
       return fail(ctx, e_ == cudaErrorMemoryAllocation ? FDF_ERR_MEM : FDF_ERR_GPU,  \
                   std::string(#call) + ": " + cudaGetErrorString(e_));               \
     }                                                                                \
@@ -304,12 +304,12 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   CUT(cudaMemcpyAsync(&err, &tc->err, 4, cudaMemcpyDeviceToHost, s));
   CUT(cudaStreamSynchronize(s));
   if (err & ERRBIT_DEGENERATE) {
-    release();
+    settle();
     return fail(ctx, FDF_ERR_USER, "Degenerate plane detected (normal vector is near zero).");
   }
   const long long m = (long long)last[0] + last[1];
   if (m == 0) {
-    release();
+    settle();
     return fail(ctx, FDF_ERR_ARG_WRONG, "fdf_LocatorTrain: the walk located none of the sample points");
   }
   mlp_make_samples(tb.x, tb.y, tb.z, tb.cell, slot, flag, n, L.norm, g, xs, ts, s);
@@ -317,7 +317,7 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   // --- training
   const int B = (int)batch;
   int r = ensure_scratch(ctx, B);
-  if (r) { release(); return r; }
+  if (r) { settle(); return r; }
   TrainScratch S = carve_scratch(L.scratch, L.batch_cap);
   CUT(cudaMemsetAsync(S.err, 0, 4, s));
   float sc[3];
@@ -345,7 +345,7 @@ int fdf_LocatorTrain(FdfContext *ctx, int64_t n_samples, uint64_t seed, int64_t 
   CUT(cudaMemcpyAsync(&errw, S.err, 4, cudaMemcpyDeviceToHost, s));
   CUT(cudaStreamSynchronize(s));
 #undef CUT
-  release();
+  settle();
   L.has_params = !(errw & ERRBIT_TC_TIMEOUT);   // weights from a step that timed out are not kept as valid
   if (errw & ERRBIT_TC_TIMEOUT) return fail(ctx, FDF_ERR_GPU, "fdf_LocatorTrain: tensor-core wait timed out");
   return FDF_SUCCESS;

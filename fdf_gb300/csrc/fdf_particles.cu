@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(128) k_interp_points(const long long *__restri
               [&](int c, double &vx, double &vy, double &vz) {
                 const int ni = (int)i + (c & 1), nj = (int)j + ((c >> 1) & 1), nk = (int)k + (c >> 2);
                 if (DIRECT) {
-                  fdfx::corner_value<0, 0, 0>(field, g, ni, nj, nk, vx, vy, vz);
+                  fdfx::corner_value<0>(field, g, ni, nj, nk, vx, vy, vz);
                 } else {
                   const double *at = field + (((long long)nk * my + nj) * mx + ni);
                   vx = __ldg(at); vy = __ldg(at + g.Nn); vz = __ldg(at + 2 * g.Nn);

@@ -51,9 +51,8 @@ __device__ __forceinline__ float2 walk_pair(double v) {
   return fdfx::split_rn(v);
 }
 
-// UpdateParticleWeights (ParticleSwarm.c:1010-1047) from the concluding cell's FP64 distances, INT of
-// each one's three products on the integer pipe.
-template <int INT>
+// UpdateParticleWeights (ParticleSwarm.c:1010-1047) from the concluding cell's FP64 distances (INT: exact_face).
+template <bool INT>
 __device__ __forceinline__ void exact_weights(const double *__restrict__ row, double x, double y, double z, double &a1,
                                               double &a2, double &a3) {
   double d[6];
@@ -70,14 +69,14 @@ __device__ __forceinline__ void exact_weights(const double *__restrict__ row, do
 
 // The step's walk.  Bound by the FP64 pipe in a large swarm (advection, the weights of the concluding
 // cell: 36 of 54 operations are its six distances) and by the walk's dependent row loads in a small one.
-// INT = 2: two of each distance's three products on the integer pipe, at 1152 resident threads; per step
+// INT: two of each distance's three products on the integer pipe, at 1152 resident threads; per step
 // in a 64 x 64 x 1024 grid 249 -> 240 us at 2M particles, 467 -> 415 at 4M, and 1848 -> 1707 at 16M in
 // 96 x 96 x 1536 (one product 1830, three 1778, two at 1024 threads 1718, at 1280 1741).  The products'
 // extra instructions lengthen each warp's chain, which a small swarm waits for: 83 -> 90 us at 500k,
-// 139 -> 143 at 1M.  So INT = 0 stays below WALK_INT_MIN slots, about ten waves of resident threads.
+// 139 -> 143 at 1M.  So INT is false below WALK_INT_MIN slots, about ten waves of resident threads.
 constexpr int WALK_INT_MIN = 3 << 19;
 
-template <int INT>
+template <bool INT>
 __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS + (INT ? 1 : 0))
     k_locate(SwarmBuf b, GridDims g, const float *__restrict__ table, const double *__restrict__ planes, double dt,
                int advect, int reset_first, const double *__restrict__ bbox, int drop_removed, DevCounters *cnt,
@@ -171,7 +170,7 @@ __global__ void __launch_bounds__(FDF_PLAIN_THREADS, FDF_PLAIN_MIN_BLOCKS)
   double a1 = 0.0, a2 = 0.0, a3 = 0.0;
   if (!lost) {
     const long long cell = ((long long)w.k * g.JM + w.j) * g.IM + w.i;
-    exact_weights<0>(planes + cell * FDF_ROW, x, y, z, a1, a2, a3);
+    exact_weights<false>(planes + cell * FDF_ROW, x, y, z, a1, a2, a3);
   }
   cell_out[3 * (size_t)p] = lost ? -1 : w.i;
   cell_out[3 * (size_t)p + 1] = lost ? -1 : w.j;
@@ -196,7 +195,7 @@ void launch_locate(const SwarmBuf &b, int n_cap, GridDims g, const float *table,
   // advect and drop_removed are both set by the fused step, which also resets statuses first
   constexpr int th = FDF_PLAIN_THREADS;
   const unsigned int blocks = n_cap > 0 ? (unsigned int)((n_cap + th - 1) / th) : 1u;
-  auto *kern = n_cap >= WALK_INT_MIN ? k_locate<2> : k_locate<0>;
+  auto *kern = n_cap >= WALK_INT_MIN ? k_locate<true> : k_locate<false>;
   kern<<<blocks, th, 0, s>>>(b, g, table, planes, dt, advect, drop_removed, bbox, drop_removed, cnt, keys, rank, count,
                              sentinel);
 }

@@ -63,17 +63,16 @@ using fdfx::sub;
 
 __device__ __forceinline__ double pair_value(float2 p) { return __dadd_rn((double)p.x, (double)p.y); }
 
-// Exact FP64 signed distance of face f (the plain path's arithmetic), thresholded.  INT: how many of its
-// three products the integer pipe makes (the same bits).
-template <int INT = 0>
+// Exact FP64 signed distance of face f (the plain path's arithmetic), thresholded.  INT: two of its three
+// products on the integer pipe (the same bits).
+template <bool INT = false>
 __device__ __forceinline__ double exact_face(const double *__restrict__ row64, int f, double x, double y, double z) {
   const double2 *r = reinterpret_cast<const double2 *>(row64);
   double2 p0 = __ldg(r + 3 * f), p1 = __ldg(r + 3 * f + 1), p2 = __ldg(r + 3 * f + 2);
   double2 tf = __ldg(r + 18);
-  const double tx = INT >= 1 ? fdfx::mul_int(sub(p0.x, x), p1.y) : mul(sub(p0.x, x), p1.y);
-  const double ty = INT >= 2 ? fdfx::mul_int(sub(p0.y, y), p2.x) : mul(sub(p0.y, y), p2.x);
-  const double tz = INT >= 3 ? fdfx::mul_int(sub(p1.x, z), p2.y) : mul(sub(p1.x, z), p2.y);
-  double dd = add(add(tx, ty), tz);
+  const double tx = INT ? fdfx::mul_int(sub(p0.x, x), p1.y) : mul(sub(p0.x, x), p1.y);
+  const double ty = INT ? fdfx::mul_int(sub(p0.y, y), p2.x) : mul(sub(p0.y, y), p2.x);
+  double dd = add(add(tx, ty), mul(sub(p1.x, z), p2.y));
   if (fdfx::abs_lt_bits(dd, fdfx::ubits(tf.x), fdfx::is_nan(tf.x))) dd = 0.0;
   return dd;
 }

@@ -279,22 +279,18 @@ MLP_FLOPS = 2 * (3 * 128 + 128 * 128 + 128 * 128 + 128 * 3)   # per particle, on
 # DRAM bytes (read + write) per launch of a stage's kernels, measured by ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum, one pass) on this workload at full size, with
 # the units the stage processed then: live particles, or guessed particles for the network and
-# the walk from the guess.  The FP32 walk and the plain form's kernels as captured before their rows were
-# swizzled and their chains changed: the same arrays read and written.
+# the walk from the guess.  Only of kernels that run as they were captured; the walks from the previous cell
+# and the plain form's have changed since and have no entry.
+_BENT = "bent_pipe_96x96x1536_n64000000_cfl4"
 TRAFFIC = {
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "advect_locate"): (7.740e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "learned_guess"): (0.598e9, "guesses", 12.92e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "guess_walk"): (2.093e9, "guesses", 12.92e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "learned_fp32", "deposit"): (1.352e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "advect_locate"): (7.623e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "fp32", "deposit"): (1.352e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "advect_locate"): (13.444e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "gather_interpolate"): (10.885e9, "particles", 63.81e6),
-    ("bent_pipe_96x96x1536_n64000000_cfl4", "plain_fp64", "deposit"): (2.651e9, "particles", 63.81e6),
+    (_BENT, "learned_fp32", "learned_guess"): (0.598e9, "guesses", 12.92e6),
+    (_BENT, "learned_fp32", "guess_walk"): (2.093e9, "guesses", 12.92e6),
+    (_BENT, "learned_fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
+    (_BENT, "learned_fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
+    (_BENT, "learned_fp32", "deposit"): (1.352e9, "particles", 63.81e6),
+    (_BENT, "fp32", "sort_by_cell"): (1.324e9, "particles", 63.81e6),
+    (_BENT, "fp32", "gather_interpolate"): (7.925e9, "particles", 63.81e6),
+    (_BENT, "fp32", "deposit"): (1.352e9, "particles", 63.81e6),
 }
 
 
@@ -305,6 +301,7 @@ def stage_traffic(wl, form: str, stage: str, n_avg: float, guesses: float):
         return None
     total, unit, units = t
     return total * ((guesses if unit == "guesses" else n_avg) / units)
+
 
 _TRAINED = {}   # workload name -> (trained parameters, training report)
 

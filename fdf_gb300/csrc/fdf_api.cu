@@ -1173,8 +1173,9 @@ int fdf_PerformInitialSetup(FdfContext *ctx, FdfStepInfo *info) {
 
 // One step on the stream, without a host round trip.  After `settled` steps since the last change of
 // anything a captured step bakes in, a step replays a CUDA graph captured for the current swarm
-// buffer parity: one launch instead of nine.  (A run of 10,000 particles with ten steps, their
-// counts read back: 1.52 ms with eager launches, 13 a step then, 1.06 ms now.)  Stage timing and a caller's own capture of the stream run it eagerly.
+// buffer parity: one launch instead of eight (plain form).  (A run of 10,000 particles with ten steps, their
+// counts read back: 1.52 ms with eager launches, 13 a step then, 1.06 ms with them replayed.)  Stage timing, a
+// caller's own capture of the stream and, in the learned form, particles that may have no cell run it eagerly.
 static int step_on_stream(FdfContext *ctx, int settled) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   CU(cudaSetDevice(ctx->device));

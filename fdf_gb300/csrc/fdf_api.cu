@@ -1276,7 +1276,7 @@ int fdf_SortByCell(const int32_t *cell_ids, int64_t n, int64_t ncells, uint32_t 
   // where there is no room for these, cursors again
   const size_t nsums = (scan_scratch_words(ncells + 1) + 63) / 64 * 64;
   unsigned int *sums = nullptr;
-  bool ranks = !cell_sort_by_tiles(n, ncells);
+  bool ranks = !cell_sort_on_cursors(n, ncells);
   if (ranks && (dev_alloc_one_fails() || cudaMallocAsync((void **)&sums, 4ull * (nsums + n), s) != cudaSuccess)) {
     (void)cudaGetLastError();
     ranks = false;

@@ -241,7 +241,7 @@ void launch_scatter_slots(const unsigned int *keys, const unsigned int *rank, in
 // lost_scratch [n_cap], also the LOST particles' bucket ncells (cnt: its barriers).  Returns the kernels launched.
 int launch_order_segments(const unsigned int *cell_start, int ncells, const long long *pid, unsigned int *perm,
                           unsigned int *lost_scratch, int n_cap, DevCounters *cnt, int num_sms, cudaStream_t s);
-bool cell_sort_by_tiles(long long n, long long ncells);   // ids counted in shared memory, on cursors
+bool cell_sort_on_cursors(long long n, long long ncells);   // cursors rather than ranks as scratch
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
                           unsigned int *cell_start, unsigned int *rank, unsigned int *cursor, unsigned int *sums,
                           cudaStream_t s);

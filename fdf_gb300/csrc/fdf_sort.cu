@@ -536,26 +536,34 @@ __global__ void __launch_bounds__(256) k_cell_rank(const int *__restrict__ cell,
 
 // A tile of TILE ids at a time, for ids nearly in order (a step's ids are: a particle moves a few cells): a block
 // whose ids span fewer than TILE_BINS cells counts them in shared memory and adds its counts to count[] cell
-// by cell -- neighbouring lanes on neighbouring words, one request where k_cell_rank makes 32.  SLOTS: the
-// second pass, which counts again, takes the block's place in each cell from `count` (the cells' cursors,
-// cell_start before) and writes the slots: nothing is kept per id between the passes, so the scratch is a
-// word per cell, a third of a word per id at most.  A block whose ids span more merges runs of equal
-// neighbours in a warp, as k_cell_rank does.  Bound by the latency of its phases: 32 registers and four
-// blocks an SM.
-// The whole sort with a rank kept per id between the passes, and now: 16M nearly sorted ids in 4M cells 191 -> 174
-// us (each call after a synchronisation, which gives the scratch back: 408 -> 333), 32M in 1M 663 -> 628 (1011 ->
-// 788), 64M in 14M 635 -> 542 (1217 -> 778); 16M in no order 393 -> 397 (608 -> 555), 32M in 1M 1339 -> 1196 (1681
-// -> 1360); 16M in runs of 8 and of 32 at random 298 -> 180 and 424 -> 218, one id in 8192 far off 249 -> 157.
-// From three ids per cell on, where a tile of ids in order spans 2731 cells and leaves the rest of the bins
-// for its disorder, and from 6M ids: against k_cell_rank and k_cell_place 102 for 118 us nearly sorted and 199 for
-// 187 in no order at 8M ids (3.1 per cell), 68 for 66 and 107 for 92 at 3.2M; at two per cell 111 for 125, 210 for
-// 202 at 8M, at one 161 for 158, 271 for 234.
+// by cell -- neighbouring lanes on neighbouring words, one request where k_cell_rank makes 32.  A block whose ids
+// span more merges runs of equal neighbours in a warp, as k_cell_rank does.
+//   RANK: rank[s] as k_cell_rank makes it, from the counts before the block's and the id's place in the block.
+//   COUNT, then SLOTS (count: the cells' cursors, cell_start before): the second pass counts again and writes the
+//   slots, so that nothing is kept per id between the passes and the scratch is a word per cell.
+// Bound by the latency of their phases: 32 registers (an id and its place share a word) and four blocks an SM.
+// The whole sort, with RANK and with COUNT and SLOTS: 16M nearly sorted ids in 4M cells 191 and 174 us (each call
+// after a synchronisation, which gives the scratch back: 408 and 333), 32M in 1M 663 and 628 (1011 and 788), 64M in
+// 14M 635 and 542 (1217 and 778); 16M in no order 393 and 397 (608 and 555); but 8M nearly sorted 100 and 104 (251
+// and 267), in no order 190 and 201, 4M 64 and 74, 111 and 128: so COUNT and SLOTS from TILE_CURSORS ids on,
+// where the ranks take 32 MB, the pool's remapping begins to tell and the ids no longer stay in L2.
+// Against k_cell_rank: from three ids per cell on, where a tile of ids in order spans 2731 cells and leaves the
+// rest of the bins for its disorder, and from 3M ids, half a wave of blocks: 3.2M nearly sorted by 64 and by 4096
+// cells 62 and 80 us against 67 and 93, 6M 80 and 116 against 93 and 137; 6M in no order 142 against 140.
+// One atomic per id where a tile spans too much took 16M ids in runs of 8 and 32 at random 298 and 424 us, now
+// 180 and 218; one id in 8192 far off 249, now 157.
 constexpr int TILE_THREADS = 512, TILE_ITEMS = 16, TILE = TILE_THREADS * TILE_ITEMS, TILE_BINS = 12224;
-constexpr long long TILE_MIN = 6 << 20;
-template <bool SLOTS>
+constexpr long long TILE_MIN = 3 << 20, TILE_CURSORS = 8 << 20;
+enum { COUNT, RANK, SLOTS };
+template <int WHAT>
 __global__ void __launch_bounds__(TILE_THREADS, 4) k_cell_tile(const int *__restrict__ cell, long long n, long long ncells,
                                                              unsigned int *__restrict__ count,
-                                                             unsigned int *__restrict__ perm) {
+                                                             unsigned int *__restrict__ out) {
+  // an id's rank (RANK) or place (SLOTS)
+  auto put = [&](long long s, unsigned int at) {
+    if (WHAT == RANK) out[s] = at;
+    else out[at] = (unsigned int)s;
+  };
   __shared__ unsigned int bin[TILE_BINS];
   __shared__ unsigned int span[2];
   const long long base = (long long)blockIdx.x * TILE + threadIdx.x;
@@ -586,11 +594,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_cell_tile(const int *__rest
     for (unsigned int b = threadIdx.x; b < bins; b += TILE_THREADS) bin[b] = 0u;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < TILE_ITEMS; ++q)   // SLOTS: from here on the bin and, above it, the id's place in it
+    for (int q = 0; q < TILE_ITEMS; ++q)   // from here on the bin and, above it, the id's place in it
       if (key[q] != 0xffffffffu) {
         key[q] -= lo;
         const unsigned int place = atomicAdd(&bin[key[q]], 1u);
-        if (SLOTS) key[q] |= place << 16;
+        if (WHAT != COUNT) key[q] |= place << 16;
       }
     __syncthreads();
 #pragma unroll 8
@@ -598,14 +606,14 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_cell_tile(const int *__rest
       const unsigned int c = bin[b];
       if (c != 0u) {
         const unsigned int before = atomicAdd(count + lo + b, c);
-        if (SLOTS) bin[b] = before;
+        if (WHAT != COUNT) bin[b] = before;
       }
     }
-    if (!SLOTS) return;
+    if (WHAT == COUNT) return;
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < TILE_ITEMS; ++q)
-      if (key[q] != 0xffffffffu) perm[bin[key[q] & 0xffffu] + (key[q] >> 16)] = (unsigned int)(base + q * TILE_THREADS);
+      if (key[q] != 0xffffffffu) put(base + q * TILE_THREADS, bin[key[q] & 0xffffu] + (key[q] >> 16));
     return;
   }
   constexpr int IN_FLIGHT = 4;
@@ -623,12 +631,11 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_cell_tile(const int *__rest
       if (leader[q] == lane && k != 0xffffffffu)
         at[q] = atomicAdd(count + k, (unsigned int)((later ? __ffs((int)later) - 1 : 32) - lane));
     }
-    if (SLOTS) {
+    if (WHAT != COUNT) {
 #pragma unroll
       for (int q = 0; q < IN_FLIGHT; ++q) {
         const unsigned int first = __shfl_sync(0xffffffffu, at[q], leader[q]);
-        if (key[h + q] != 0xffffffffu)
-          perm[first + (unsigned int)(lane - leader[q])] = (unsigned int)(base + (h + q) * TILE_THREADS);
+        if (key[h + q] != 0xffffffffu) put(base + (h + q) * TILE_THREADS, first + (unsigned int)(lane - leader[q]));
       }
     }
   }
@@ -727,27 +734,30 @@ int launch_order_segments(const unsigned int *cell_start, int ncells, const long
   return 2;
 }
 
-bool cell_sort_by_tiles(long long n, long long ncells) { return n >= TILE_MIN && n >= 3 * ncells; }
+static bool by_tiles(long long n, long long ncells) { return n >= TILE_MIN && n >= 3 * ncells; }
+
+bool cell_sort_on_cursors(long long n, long long ncells) { return by_tiles(n, ncells) && n >= TILE_CURSORS; }
 
 // Stable counting sort of particle slots by cell id, on caller-provided scratch: sums
-// [scan_scratch_words(ncells + 1)] and cursor [ncells] or, where cell_sort_by_tiles does not hold, rank [n]
-// (with a cursor the slots then come from a second pass of atomics).  cell_start [ncells + 1] is both the
-// histogram and (after the scan) the output.
+// [scan_scratch_words(ncells + 1)] and either rank [n] (and no cursor), for sizes where cell_sort_on_cursors does
+// not hold, or cursor [ncells] (the slots then come from a second pass of atomics).  cell_start [ncells + 1] is
+// both the histogram and (after the scan) the output.
 void cell_sort_on_scratch(const int *cell, long long n, long long ncells, unsigned int *perm,
                           unsigned int *cell_start, unsigned int *rank, unsigned int *cursor, unsigned int *sums,
                           cudaStream_t s) {
   const int th = 256;
   const unsigned int blocks = (unsigned int)std::max<long long>((n + th - 1) / th, 1);
   const unsigned int blocks_items = (blocks + SORT_ITEMS - 1) / SORT_ITEMS, tiles = (unsigned int)((n + TILE - 1) / TILE);
-  const bool by_tiles = cursor && cell_sort_by_tiles(n, ncells);
+  const bool tiled = by_tiles(n, ncells);
   cudaMemsetAsync(cell_start, 0, 4ull * (ncells + 1), s);
-  if (by_tiles) k_cell_tile<false><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cell_start, nullptr);
+  if (tiled && rank) k_cell_tile<RANK><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cell_start, rank);
+  else if (tiled) k_cell_tile<COUNT><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cell_start, nullptr);
   else if (rank) k_cell_rank<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank);
   else k_cell_histogram<<<blocks, th, 0, s>>>(cell, n, ncells, cell_start);
   exclusive_scan_u32(cell_start, ncells + 1, sums, s);
   if (cursor) cudaMemcpyAsync(cursor, cell_start, 4ull * ncells, cudaMemcpyDeviceToDevice, s);
-  if (by_tiles) k_cell_tile<true><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cursor, perm);
-  else if (rank) k_cell_place<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank, perm);
+  if (rank) k_cell_place<<<blocks_items, th, 0, s>>>(cell, n, ncells, cell_start, rank, perm);
+  else if (tiled) k_cell_tile<SLOTS><<<tiles, TILE_THREADS, 0, s>>>(cell, n, ncells, cursor, perm);
   else k_cell_slots<<<blocks, th, 0, s>>>(cell, n, ncells, cursor, perm);
   launch_order_segments(cell_start, (int)ncells, nullptr, perm, nullptr, 0, nullptr, 0, s);
 }

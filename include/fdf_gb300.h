@@ -262,9 +262,9 @@ int fdf_DepositKFaceLayer(FdfContext *ctx, int64_t k, const double *seed, const 
  * first sorted slot of cell c (cell_start[ncells] = number of placed slots) and
  * perm[cell_start[c] .. cell_start[c+1]) lists cell c's slot indices in ascending
  * order.  Scratch is stream-ordered (cudaMallocAsync/cudaFreeAsync on `stream`): a word per
- * cell from 6M ids and three per cell on, else a word per id or, where the device has no room
+ * cell from 8M ids and three per cell on, else a word per id or, where the device has no room
  * for that, per cell.  The device's pool keeps it until the next synchronisation, after
- * which a call maps it anew (150 us, from 64 MB on more).
+ * which a call maps it anew (150 us, from 32 MB on more).
  * No counterpart call in the reference, which keeps DMSwarm in insertion order; it
  * is the sort-by-cell step that makes the gathers of this library coalesced. */
 int fdf_SortByCell(const int32_t *cell_ids, int64_t n, int64_t ncells, uint32_t *perm, uint32_t *cell_start,

@@ -11,11 +11,13 @@ from tests.test_gpu_sort import reference, sort_by_cell_gpu
 
 pytestmark = pytest.mark.gpu
 
-N = 6 << 20
+N = 8 << 20   # from here on a second count instead of ranks
+RANKS = 3 << 20   # from here on tiles
 TILE, BINS = 8192, 12224
 
 
-@pytest.mark.parametrize("n,ncells", [(N - 1, 90_000), (N, 90_000), (N + 77, N // 3), (N + 77, N // 3 + 1000), (N + TILE, 700_000)])
+@pytest.mark.parametrize("n,ncells", [(N - 1, 90_000), (N, 90_000), (N + 77, N // 3), (N + 77, N // 3 + 1000), (N + TILE, 700_000),
+                                      (RANKS - 1, 40_000), (RANKS + 5, 40_000), (RANKS + TILE, RANKS // 3)])
 def test_tiles_of_every_kind(require_gpu, n, ncells):
     rng = np.random.default_rng(n + ncells)
     cells = np.arange(n, dtype=np.int64) * ncells // n + rng.integers(-500, 501, n)   # some below zero or past the last
@@ -67,10 +69,11 @@ def test_scratch_is_a_word_per_cell(require_gpu):
     assert 0 < used.value < 4.5 * 1_000_000
 
 
-def test_runs_of_equal_ids_with_far_jumps(require_gpu):
-    """One atomic per id took these twice the time of the way without tiles, one per run of a warp as much."""
+@pytest.mark.parametrize("n", [16_000_000, 6_000_000])
+def test_runs_of_equal_ids_with_far_jumps(require_gpu, n):
+    """One atomic per id took these twice the time of the way without tiles, one per run of a warp as much (16M: a second
+    count; 6M: ranks)."""
     import torch
-    n = 16_000_000
     g = torch.Generator(device="cuda").manual_seed(1)
     ids = torch.randint(0, n // 4, (n // 32,), device="cuda", generator=g).repeat_interleave(32).to(torch.int32).contiguous()
     took = []

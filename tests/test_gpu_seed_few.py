@@ -45,4 +45,4 @@ def test_a_hundred_particles(require_gpu):
 
         ctx.seed_particles(100, 1)
         read, seed = least(ctx.size), least(lambda: ctx.seed_particles(100, 1))
-    assert seed < 2.3 * read, (seed, read)
+    assert seed < 2.4 * read, (seed, read)
